@@ -80,11 +80,11 @@ typedef struct tcpxbUnpackOpts {
   uint32_t flag_value;
   uint32_t* ticket;
   int max_ctas;            // 0 = one CTA per SM
-  // Programmatic dependent launch: when non-zero the launch may be scheduled while the
-  // previous kernel of the stream is still running; its CTAs become resident as SMs free
-  // up, set up their barriers, and wait for that kernel to complete (and its writes to
-  // be visible) before they touch any memory.  Results are the same; back-to-back
-  // launches lose the gap between kernels.
+  // Programmatic dependent launch: the launch may be scheduled while the previous kernel
+  // of the stream is still running; its CTAs become resident as SMs free up, set up
+  // their barriers, and wait for that kernel to complete (and its writes to be visible)
+  // before they touch any memory.  Every launch is made that way; the field is accepted
+  // for callers that ask for it.
   int early_launch;
 } tcpxbUnpackOpts;
 
@@ -144,6 +144,13 @@ int tcpxb_wait_flags(const uint32_t* flags, int n, uint32_t value, uint64_t wait
 // Writes `value` (release, system scope) to each peer_flags[i]: "my buffers are
 // ready for epoch `value`".  The counterpart of tcpxb_wait_flags.
 int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void* stream);
+
+// Copies `bytes` from device memory to mapped host memory and then writes `value` to
+// *flag (release, system scope; mapped host memory too): a small message's way to its
+// staging buffer, in stream order and without the copy engine.  `ticket` is one
+// zero-initialised uint32 on the launching GPU; the kernel leaves it zero.
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket,
+                    uint32_t* flag, uint32_t value, void* stream);
 
 // Intra-node reduce-scatter stage over peer memory: out[i] = sum over r of
 // srcs[r][shard_off + i], element-wise, for `bytes` bytes.  srcs are peer-mapped

@@ -246,6 +246,14 @@ int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void*
   return TCPXB_K_OK;
 }
 
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value, void*) {
+  if (flag == nullptr || ticket == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
+    return fail(TCPXB_K_INVALID, "null source, destination, ticket or flag");
+  if (tcpxb::gpu::standinMovesData()) memcpy(host_dst, src, bytes);
+  __atomic_store_n(flag, value, __ATOMIC_RELEASE);
+  return TCPXB_K_OK;
+}
+
 int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_off, uint64_t bytes, int dtype, void*) {
   if (out == nullptr || srcs == nullptr || nsrcs < 1 || nsrcs > TCPXB_MAX_PEERS) return fail(TCPXB_K_INVALID, "bad source list");
   if (dtype != TCPXB_BF16 && dtype != TCPXB_F32) return fail(TCPXB_K_INVALID, "reduce needs bf16 or f32");

@@ -78,11 +78,12 @@ struct UnpackParams {
 };
 
 struct SlotInfo {
-  uint32_t src_off;
-  uint32_t len;
+  uint64_t src_off;
   uint64_t dst_off;
-  uint32_t bulk;   // bytes moved by the bulk path (multiple of 16, may be 0)
-  uint32_t pad[3];
+  uint32_t len;
+  uint32_t bulk;     // bytes moved by the bulk path (multiple of 16, may be 0)
+  uint32_t shifted;  // what the bulk path leaves of the fragment is in shared memory too
+  uint32_t index;    // record
 };
 
 // ---------------------------------------------------------------- PTX wrappers
@@ -185,6 +186,48 @@ __device__ __forceinline__ uint4 ld_volatile_v4(const void* p) {
                : "memory");
   return v;
 }
+// Weak and not through the read-only path: with programmatic dependent launch a kernel's lifetime
+// begins before its predecessor's writes are visible, so nothing may be assumed constant over it.
+__device__ __forceinline__ uint4 ld_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_v4_hint(const void* p, uint64_t policy) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p), "l"(policy)
+               : "memory");
+  return v;
+}
+struct Vec32 { uint4 lo, hi; };
+__device__ __forceinline__ Vec32 ld_v8(const void* p) {
+  Vec32 v;
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ Vec32 ld_v8_evict_first(const void* p) {
+  Vec32 v;
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_v8(void* p, const Vec32& v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z),
+               "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y), "r"(v.hi.z), "r"(v.hi.w)
+               : "memory");
+}
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v) {
   asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -267,11 +310,23 @@ __device__ __forceinline__ void copy_units(const uint8_t* src, const UnpackParam
   }
 }
 
+// Why a record is skipped (TCPXB_ST_OK: it is not).
+template <int RED>
+__device__ __forceinline__ uint32_t refused(const UnpackParams& p, uint32_t src_off, uint32_t len, uint64_t dst_off) {
+  if ((uint64_t)src_off + len > p.pool_bytes || dst_off + len > p.dst_bytes || dst_off + len < dst_off) return TCPXB_ST_BOUNDS;
+  if (RED != TCPXB_U8) {
+    constexpr uint32_t es = (RED == TCPXB_BF16) ? 2 : 4;
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p.pool + src_off) | reinterpret_cast<uintptr_t>(p.dst + dst_off) |
+                        reinterpret_cast<uintptr_t>(p.acc + dst_off) | len;
+    if ((a & (es - 1)) != 0) return TCPXB_ST_ALIGN;
+  }
+  return TCPXB_ST_OK;
+}
+
 // Warp-cooperative generic path for `n` bytes of any alignment: plain loads and
 // stores, widest unit the common alignment of source and destination allows.
 template <int RED, bool L2RED, int FAN>
-__device__ void warp_generic(const UnpackParams& p, uint32_t src_off, uint64_t dst_off, uint32_t n,
-                             uint32_t desc_index, int lane, uint32_t* cta_err) {
+__device__ void warp_generic(const UnpackParams& p, uint64_t src_off, uint64_t dst_off, uint32_t n, int lane) {
   if (n == 0) return;
   const uint8_t* src = p.pool + src_off;
   const int fan = (FAN != FAN_NONE);
@@ -298,13 +353,6 @@ __device__ void warp_generic(const UnpackParams& p, uint32_t src_off, uint64_t d
     }
   } else {
     constexpr uint32_t es = (RED == TCPXB_BF16) ? 2 : 4;
-    uintptr_t s = reinterpret_cast<uintptr_t>(src);
-    uintptr_t d = reinterpret_cast<uintptr_t>(p.dst + dst_off);
-    uintptr_t a = reinterpret_cast<uintptr_t>(p.acc + dst_off);
-    if (((s | d | a | n) & (es - 1)) != 0) {
-      if (lane == 0) { report(p.status, TCPXB_ST_ALIGN, desc_index); atomicOr(cta_err, 1u); }
-      return;
-    }
     uint32_t elems = n / es;
     for (uint32_t i = lane; i < elems; i += 32) {
       uint64_t off = dst_off + (uint64_t)i * es;
@@ -340,44 +388,84 @@ __device__ void warp_generic(const UnpackParams& p, uint32_t src_off, uint64_t d
   }
 }
 
+// Four bytes at any byte offset of shared memory, from the two words they straddle.
+__device__ __forceinline__ uint32_t word_at(const uint8_t* base, uint32_t byte_off) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(base + (byte_off & ~3u));
+  return __funnelshift_r(w[0], w[1], (byte_off & 3u) * 8);
+}
+
+// A fragment whose source (and accumulator) lie in shared memory at a phase of their own: `src` and
+// `acc` point at its first byte.  The warp writes whole destination words, 128 bytes per store
+// instruction; bytes before the first and behind the last word go one element at a time.
+template <int RED, int FAN>
+__device__ __forceinline__ void store_shifted(const UnpackParams& p, const uint8_t* sbase, uint32_t sphase, const uint8_t* abase,
+                                              uint32_t aphase, uint64_t dst_off, uint32_t n, int lane) {
+  const int fan = (FAN != FAN_NONE);
+  uint32_t head = static_cast<uint32_t>((4 - (reinterpret_cast<uintptr_t>(p.dst + dst_off) & 3)) & 3);
+  if (head > n) head = n;
+  const uint32_t words = (n - head) >> 2;
+#pragma unroll 4
+  for (uint32_t i = lane; i < words; i += 32) {
+    const uint32_t o = head + (i << 2);
+    uint32_t v = word_at(sbase, sphase + o);
+    if (RED == TCPXB_BF16) v = add_bf16x2(word_at(abase, aphase + o), v);
+    if (RED == TCPXB_F32) v = __float_as_uint(__uint_as_float(word_at(abase, aphase + o)) + __uint_as_float(v));
+    store_all<uint32_t>(p.dst, p, fan, dst_off + o, v);
+  }
+  // at most three bytes on either side: lanes 0.. take the head, lanes 4.. the tail
+  constexpr uint32_t es = RED == TCPXB_U8 ? 1 : 2;
+  const uint32_t tail0 = head + (words << 2);
+  const uint32_t o = lane < 4 ? lane * es : tail0 + (lane - 4) * es;
+  if (RED != TCPXB_F32 && (lane < 4 ? o < head : (lane < 8 && o < n))) {
+    if (RED == TCPXB_U8) {
+      store_all<uint8_t>(p.dst, p, fan, dst_off + o, sbase[sphase + o]);
+    } else {
+      const float x = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sbase + sphase + o));
+      const float y = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(abase + aphase + o));
+      store_all<__nv_bfloat16>(p.dst, p, fan, dst_off + o, __float2bfloat16_rn(x + y));
+    }
+  }
+}
+
 // ------------------------------------------------------------------ the kernel
 template <int RED, bool L2RED, int FAN>
 struct Cfg {
   static constexpr bool kAccSlot = (RED != TCPXB_U8) && !L2RED;
-  static constexpr int kStride = kAccSlot ? 2 * kSlot : kSlot;
+  // A slot holds a fragment and the up to 15 bytes on either side that complete its 16-byte vectors.
+  static constexpr int kSlotBytes = kSlot + 16;
+  static constexpr int kStride = kAccSlot ? 2 * kSlotBytes : kSlotBytes;
   static constexpr int kDepth = kAccSlot ? TCPXB_DEPTH_REDUCE : TCPXB_DEPTH_COPY;
-  static_assert(kWarps * kDepth * kStride + kWarps * kDepth * 40 <= 227 * 1024, "slot rings must fit one CTA's shared memory");
   static constexpr int kDataBytes = kWarps * kDepth * kStride;
   static constexpr int kSmemBytes = kDataBytes + kWarps * kDepth * (8 + (int)sizeof(SlotInfo));
+  static_assert(kSmemBytes + 1024 <= 227 * 1024, "slot rings must fit one CTA's shared memory");
 };
 
 template <int RED, bool L2RED, int FAN>
 __global__ void __launch_bounds__(kThreads, 1)
 unpack_kernel(const __grid_constant__ UnpackParams p) {
   using C = Cfg<RED, L2RED, FAN>;
-  constexpr int D = C::kDepth;
   extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  uint8_t* wbuf = smem + warp * D * C::kStride;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kDataBytes) + warp * D;
-  SlotInfo* infos = reinterpret_cast<SlotInfo*>(smem + C::kDataBytes + kWarps * D * 8) + warp * D;
+  constexpr uint32_t D = (uint32_t)C::kDepth;
+  constexpr uint32_t half = (uint32_t)C::kSlotBytes;  // one slot, or the fragment half of a pair
+  constexpr uint32_t stride = (uint32_t)C::kStride;
+  uint8_t* wbuf = smem + warp * C::kDepth * C::kStride;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kDataBytes) + warp * C::kDepth;
+  SlotInfo* infos = reinterpret_cast<SlotInfo*>(smem + C::kDataBytes + kWarps * C::kDepth * 8) + warp * C::kDepth;
 
   // Programmatic dependent launch, both roles.  As the earlier kernel: let a dependent
   // launch be scheduled from now on (its CTAs still need this one's shared memory to
   // be released before they fit).  As the later kernel: everything up to the wait
   // below touches only this CTA's shared memory; the wait returns when the previous
-  // kernel of the stream has completed and its writes are visible (at once when the
-  // launch did not ask for an early start).
-  asm volatile("griddepcontrol.launch_dependents;");
+  // kernel of the stream has completed and its writes are visible.
+  pdl_launch_dependents();
   __shared__ uint32_t cta_err;  // any warp of this CTA recorded an error
   if (threadIdx.x == 0) cta_err = 0;
-  if (lane == 0) {
-    for (int s = 0; s < D; ++s) mbar_init(smem_u32(&bars[s]), 1);
-    fence_mbar_init();
-  }
+  if (lane < (int)D) mbar_init(smem_u32(&bars[lane]), 1);
+  fence_mbar_init();
   __syncthreads();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   auto record = [&](uint32_t code, uint32_t index) {  // one lane calls this
     report(p.status, code, index);
     atomicOr(&cta_err, 1u);
@@ -435,7 +523,7 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
       const uint32_t blk = k >> 5;
       if (blk != cached_blk) {
         const uint32_t kk = (blk << 5) + lane;
-        if (kk < n) cached = __ldg(reinterpret_cast<const uint4*>(&p.descs[gw + (uint64_t)kk * G]));
+        if (kk < n) cached = ld_v4(&p.descs[gw + (uint64_t)kk * G]);
         cached_blk = blk;
       }
       so = __shfl_sync(0xffffffffu, cached.x, k & 31);
@@ -445,23 +533,40 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
     }
     const uint64_t dof = (static_cast<uint64_t>(dhi) << 32) | dlo;
     if (dead) ln = 0;
-    if ((uint64_t)so + ln > p.pool_bytes || dof + ln > p.dst_bytes || dof + ln < dof) {
-      if (lane == 0) record(TCPXB_ST_BOUNDS, idx);
+    const uint32_t bad = refused<RED>(p, so, ln, dof);
+    if (bad != TCPXB_ST_OK) {
+      if (lane == 0) record(bad, idx);
       ln = 0;
     }
-    uintptr_t al = reinterpret_cast<uintptr_t>(p.pool + so) | reinterpret_cast<uintptr_t>(p.dst + dof);
-    if (C::kAccSlot) al |= reinterpret_cast<uintptr_t>(p.acc + dof);
-    const uint32_t bulk = ((al & 15) == 0 && ln <= (uint32_t)kSlot) ? (ln & ~15u) : 0u;
+    const uintptr_t sa = reinterpret_cast<uintptr_t>(p.pool + so);
+    const uintptr_t aa = reinterpret_cast<uintptr_t>(p.acc + dof);
+    uintptr_t al = sa | reinterpret_cast<uintptr_t>(p.dst + dof);
+    if (C::kAccSlot) al |= aa;
+    const bool fits = ln <= (uint32_t)kSlot;
+    const uint32_t bulk = ((al & 15) == 0 && fits) ? (ln & ~15u) : 0u;
+    // off the 16-byte phase, or with a ragged end: that part is stored by the warp out of shared memory
+    const bool shifted = !L2RED && ((al | ln) & 15) != 0 && fits && ln != 0;
     if (lane == 0) {
       infos[slot].src_off = so;
-      infos[slot].len = ln;
       infos[slot].dst_off = dof;
+      infos[slot].len = ln;
       infos[slot].bulk = bulk;
+      infos[slot].shifted = shifted;
+      infos[slot].index = idx;
       const uint32_t bar = smem_u32(&bars[slot]);
-      if (bulk) {
+      const uint32_t sm = smem_u32(wbuf + slot * stride);
+      if (shifted) {
+        // the 16-byte vectors that hold the fragment: they reach at most 15 bytes beyond it on either
+        // side, inside the same aligned vector and so inside the same allocation
+        const uint32_t sbytes = ((uint32_t)(sa & 15) + ln + 15u) & ~15u;
+        const uint32_t abytes = C::kAccSlot ? (((uint32_t)(aa & 15) + ln + 15u) & ~15u) : 0u;
+        mbar_expect_tx(bar, sbytes + abytes);
+        bulk_g2s_hint(sm, reinterpret_cast<const void*>(sa & ~(uintptr_t)15), sbytes, bar, pool_policy);
+        if (C::kAccSlot) bulk_g2s(sm + half, reinterpret_cast<const void*>(aa & ~(uintptr_t)15), abytes, bar);
+      } else if (bulk) {
         mbar_expect_tx(bar, C::kAccSlot ? 2 * bulk : bulk);
-        bulk_g2s_hint(smem_u32(wbuf + slot * C::kStride), p.pool + so, bulk, bar, pool_policy);
-        if (C::kAccSlot) bulk_g2s(smem_u32(wbuf + slot * C::kStride + kSlot), p.acc + dof, bulk, bar);
+        bulk_g2s_hint(sm, p.pool + so, bulk, bar, pool_policy);
+        if (C::kAccSlot) bulk_g2s(sm + half, p.acc + dof, bulk, bar);
       } else {
         mbar_arrive(bar);
       }
@@ -469,7 +574,7 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
     __syncwarp();
   };
 
-  const uint32_t pro = n < (uint32_t)D ? n : (uint32_t)D;
+  const uint32_t pro = n < D ? n : D;
   for (uint32_t k = 0; k < pro && !dead; ++k) issue(k);  // a wait that ran out is not repeated for the next slot
 
   for (uint32_t k = 0; k < n; ++k) {
@@ -480,16 +585,16 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
     const uint32_t parity = (k / D) & 1;
     const uint32_t bar = smem_u32(&bars[slot]);
     if (!mbar_wait_bounded(bar, parity, dead ? (wait_ns >> 3) + 1 : wait_ns)) {
-      if (lane == 0 && !dead) record(TCPXB_ST_TIMEOUT, gw + k * G);
+      if (lane == 0 && !dead) record(TCPXB_ST_TIMEOUT, infos[slot].index);
       dead = true;
     }
     dead = __any_sync(0xffffffffu, dead);
     const SlotInfo info = infos[slot];
-    uint8_t* sfrag = wbuf + slot * C::kStride;
+    uint8_t* sfrag = wbuf + slot * stride;
     uint8_t* sout = sfrag;
     if (info.bulk && !dead) {
       if (C::kAccSlot) {
-        sout = sfrag + kSlot;
+        sout = sfrag + half;
         const uint32_t vecs = info.bulk >> 4;
         for (uint32_t i = lane; i < vecs; i += 32) {
           uint4 a = *reinterpret_cast<const uint4*>(sfrag + (i << 4));
@@ -536,9 +641,16 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
     // An (often empty) group per iteration keeps "all but the newest group" equal
     // to "every store of the iterations before this one".
     if (lane == 0) bulk_commit();
-    if (info.len > info.bulk && !dead) {
-      warp_generic<RED, L2RED, FAN>(p, info.src_off + info.bulk, info.dst_off + info.bulk,
-                                    info.len - info.bulk, gw + k * G, lane, &cta_err);
+    if (!dead) {
+      if (!L2RED && info.shifted) {
+        // all of the fragment, or the up to 15 bytes behind its last whole vector
+        store_shifted<RED, FAN>(p, sfrag + info.bulk, (uint32_t)(reinterpret_cast<uintptr_t>(p.pool + info.src_off) & 15),
+                                sfrag + half + info.bulk, (uint32_t)(reinterpret_cast<uintptr_t>(p.acc + info.dst_off) & 15),
+                                info.dst_off + info.bulk, info.len - info.bulk, lane);
+        __syncwarp();
+      } else if (info.len > info.bulk) {
+        warp_generic<RED, L2RED, FAN>(p, info.src_off + info.bulk, info.dst_off + info.bulk, info.len - info.bulk, lane);
+      }
     }
     // Refill the slot of the previous iteration: its store has had one iteration
     // to read shared memory, so this wait rarely blocks.
@@ -550,8 +662,9 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
   }
   if (lane == 0) bulk_wait_all();
 
-  if (FAN != FAN_NONE && p.flag_value != 0 && p.ticket != nullptr) {
-    // Publish completion to the peers once every CTA's stores are done.
+  if (p.flag_value != 0 && p.ticket != nullptr) {
+    // Publish completion (to the peers, or to a host that watches a mapped word) once every
+    // CTA's stores are done.
     // The ticket counts CTAs in its low half and CTAs with errors in its high half.
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -571,10 +684,145 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
   }
 }
 
+// ------------------------------------------------------------ long scatter lists
+// The 16 bytes that start `4 * word + shift / 8` bytes into a:b.
+__device__ __forceinline__ uint4 take_vec(const uint4& a, const uint4& b, uint32_t word, uint32_t shift) {
+  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (word & 2) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+  }
+  if (word & 1) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+  }
+  return make_uint4(__funnelshift_r(w[0], w[1], shift), __funnelshift_r(w[1], w[2], shift), __funnelshift_r(w[2], w[3], shift),
+                    __funnelshift_r(w[3], w[4], shift));
+}
+
+// K1 and K2 for lists of more records than the ring kernel has warps (wide_from below): one warp per record, through
+// registers, as many CTAs as that takes.  What bounds it is HBM; what it saves against the ring kernel is the
+// last, part-filled round of a persistent grid (the hardware hands a finished SM its next CTA) and, for
+// fragments off the 16-byte phase, the trip through shared memory: a warp shifts its vectors into the
+// destination's phase with lane exchanges.  A whole aligned page goes as 32-byte loads and stores; 4 x 16 bytes
+// per lane are in flight per step, which leaves room for 32 warps per SM (24 in the reduce).  Steps of 8 x 16
+// bytes are as fast on whole pages, but half of one is wasted on a 1448-byte fragment (10.5 against 7.8 us).
+// Measured inside CUDA graphs, ring kernel -> this one: copy of 64 MiB in pages 24.2 -> 23.0 us (0.87 -> 0.91 of the
+// measured copy rate), reduce 33.6 -> 31.8 us; 16 MiB in 1448-byte fragments 10.0 -> 7.6 us.
+constexpr int kWideThreads = 256;
+constexpr int kWideWarps = kWideThreads / 32;
+constexpr int kWideUnroll = 4;
+template <int RED>
+__global__ void __launch_bounds__(kWideThreads, RED == TCPXB_U8 ? 4 : 3)
+unpack_wide_kernel(const __grid_constant__ UnpackParams p) {
+  constexpr int U = kWideUnroll;
+  constexpr uint32_t es = RED == TCPXB_U8 ? 1 : RED == TCPXB_BF16 ? 2 : 4;
+  const int lane = threadIdx.x & 31;
+  const uint32_t idx = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // neighbours in the list go to different SMs
+  pdl_launch_dependents();
+  const uint64_t pool_policy = policy_evict_first();
+  if (idx >= p.count) return;
+  pdl_wait();
+  const uint4 d = ld_v4(&p.descs[idx]);
+  const uint32_t n = d.y;
+  const uint64_t dof = (static_cast<uint64_t>(d.w) << 32) | d.z;
+  const uint32_t bad = refused<RED>(p, d.x, n, dof);
+  if (bad != TCPXB_ST_OK) {
+    if (lane == 0) report(p.status, bad, idx);
+    return;
+  }
+  const uint8_t* s = p.pool + d.x;
+  const uint8_t* a = p.acc + dof;
+  uint8_t* t = p.dst + dof;
+  const uintptr_t phases = reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(t) | (RED ? reinterpret_cast<uintptr_t>(a) : 0);
+  if (n == (uint32_t)kSlot && (phases & 31) == 0) {
+#pragma unroll
+    for (int h = 0; h < kSlot / (U * 512); ++h) {
+      Vec32 v[U / 2], c[U / 2];
+      const uint32_t off = h * U * 512 + lane * 32;
+#pragma unroll
+      for (int u = 0; u < U / 2; ++u) v[u] = ld_v8_evict_first(s + off + u * 1024);
+      if (RED) {
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) c[u] = ld_v8(a + off + u * 1024);
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) {
+          v[u].lo = add_vec<RED>(c[u].lo, v[u].lo);
+          v[u].hi = add_vec<RED>(c[u].hi, v[u].hi);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U / 2; ++u) st_v8(t + off + u * 1024, v[u]);
+    }
+    return;
+  }
+  if (RED && ((reinterpret_cast<uintptr_t>(a) ^ reinterpret_cast<uintptr_t>(t)) & 15) != 0) {
+    warp_generic<RED, false, FAN_NONE>(p, d.x, dof, n, lane);  // accumulator and output in different phases
+    return;
+  }
+  // whole destination vectors, and up to 15 bytes on either side: one element each for lanes 0.. and 16..
+  uint32_t head = static_cast<uint32_t>((16 - (reinterpret_cast<uintptr_t>(t) & 15)) & 15);
+  if (head > n) head = n;
+  const uint32_t vecs = (n - head) >> 4;
+  const uint32_t q = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s + head) & 15);
+  const uint32_t edge = lane < 16 ? lane * es : head + (vecs << 4) + (lane - 16) * es;
+  const bool has_edge = lane < 16 ? edge < head : edge < n;
+  uint32_t ev = 0, ea = 0;
+  if (has_edge) {
+    if (RED == TCPXB_U8) ev = s[edge];
+    if (RED == TCPXB_BF16) { ev = *reinterpret_cast<const uint16_t*>(s + edge); ea = *reinterpret_cast<const uint16_t*>(a + edge); }
+    if (RED == TCPXB_F32) { ev = *reinterpret_cast<const uint32_t*>(s + edge); ea = *reinterpret_cast<const uint32_t*>(a + edge); }
+  }
+  const uint8_t* sv = s + head - q;  // aligned; with q != 0 the vectors are taken out of one more source vector
+  const uint32_t loads = vecs + (q != 0 && vecs != 0 ? 1 : 0);
+  for (uint32_t base = 0; base < vecs; base += 32 * U) {
+    uint4 v[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + u * 32 + lane;
+      v[u] = i < loads ? ld_v4_hint(sv + ((uint64_t)i << 4), pool_policy) : make_uint4(0, 0, 0, 0);
+    }
+    if (RED) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t i = base + u * 32 + lane;
+        c[u] = i < vecs ? ld_v4(a + head + ((uint64_t)i << 4)) : make_uint4(0, 0, 0, 0);
+      }
+    }
+    if (q != 0) {
+      const uint32_t after = base + 32 * U;  // the vector behind this step's last
+      const uint4 beyond = after < loads ? ld_v4_hint(sv + ((uint64_t)after << 4), pool_policy) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint4& nb = u + 1 < U ? v[u + 1 < U ? u + 1 : u] : beyond;
+        uint4 next = make_uint4(__shfl_down_sync(0xffffffffu, v[u].x, 1), __shfl_down_sync(0xffffffffu, v[u].y, 1),
+                                __shfl_down_sync(0xffffffffu, v[u].z, 1), __shfl_down_sync(0xffffffffu, v[u].w, 1));
+        const uint4 wrap = make_uint4(__shfl_sync(0xffffffffu, nb.x, 0), __shfl_sync(0xffffffffu, nb.y, 0),
+                                      __shfl_sync(0xffffffffu, nb.z, 0), __shfl_sync(0xffffffffu, nb.w, 0));
+        if (lane == 31) next = wrap;
+        v[u] = take_vec(v[u], next, q >> 2, (q & 3) * 8);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + u * 32 + lane;
+      if (i < vecs) *reinterpret_cast<uint4*>(t + head + ((uint64_t)i << 4)) = RED ? add_vec<RED>(c[u], v[u]) : v[u];
+    }
+  }
+  if (has_edge) {
+    if (RED == TCPXB_U8) t[edge] = static_cast<uint8_t>(ev);
+    if (RED == TCPXB_BF16)
+      *reinterpret_cast<__nv_bfloat16*>(t + edge) = __float2bfloat16_rn(__uint_as_float(ev << 16) + __uint_as_float(ea << 16));
+    if (RED == TCPXB_F32) *reinterpret_cast<float*>(t + edge) = __uint_as_float(ev) + __uint_as_float(ea);
+  }
+}
+
 // Bounded wait for peer completion flags; one warp, lane i watches flags[i].
 __global__ void wait_flags_kernel(const uint32_t* flags, int n, uint32_t value, uint64_t wait_ns,
                                   uint32_t* status) {
+  // A kernel behind this one is let in only at its end: it would hold SMs while this one waits for a peer.
   const int i = threadIdx.x;
+  pdl_wait();
   if (i >= n) return;
   uint64_t t0 = globaltimer_ns();
   for (;;) {
@@ -595,9 +843,34 @@ struct SignalParams {
 };
 __global__ void signal_flags_kernel(const __grid_constant__ SignalParams p) {
   const int i = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i < p.n && p.flags[i] != nullptr) {
     __threadfence_system();
     st_release_sys(p.flags[i], p.value);
+  }
+}
+
+// Device memory -> mapped host memory, then a flag.  Bound by the PCIe write latency at these sizes
+// (up to 64 KiB): 4 KiB per CTA, one 16-byte vector per thread, all of them posted at once.
+constexpr int kStageThreads = 256;
+__global__ void __launch_bounds__(kStageThreads)
+stage_out_kernel(const uint8_t* src, uint8_t* dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value) {
+  const uint64_t stride = (uint64_t)gridDim.x * kStageThreads;
+  const uint64_t tid = (uint64_t)blockIdx.x * kStageThreads + threadIdx.x;
+  const uint64_t vecs = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? bytes >> 4 : 0;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (uint64_t i = tid; i < vecs; i += stride) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+  for (uint64_t i = (vecs << 4) + tid; i < bytes; i += stride) dst[i] = src[i];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    if (gridDim.x == 1 || atomicAdd(ticket, 1u) == gridDim.x - 1) {
+      if (gridDim.x != 1) *ticket = 0;
+      __threadfence_system();
+      st_release_sys(flag, value);
+    }
   }
 }
 
@@ -612,6 +885,8 @@ struct PeerReduceParams {
 template <int RED>
 __global__ void __launch_bounds__(256) peer_reduce_kernel(const __grid_constant__ PeerReduceParams p) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  pdl_launch_dependents();
+  pdl_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.vecs; i += stride) {
     const uint64_t off = p.shard_off + (i << 4);
     uint4 v[TCPXB_MAX_PEERS + 1];
@@ -667,6 +942,8 @@ struct CsumScratch {
 };
 __global__ void __launch_bounds__(kCsumThreads)
 checksum_kernel(const uint8_t* buf, uint64_t bytes, uint64_t* out, CsumScratch* scratch) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint64_t words = bytes >> 2;
   const uint32_t* w = reinterpret_cast<const uint32_t*>(buf);
   uint64_t sum = 0;
@@ -787,8 +1064,27 @@ int deviceInfo(int* dev_out) {
   return TCPXB_K_OK;
 }
 
+// Every launch may be scheduled while its predecessor in the stream still runs (programmatic
+// dependent launch): the kernels wait for that predecessor on the device before they touch any
+// memory, so results do not change and back-to-back launches lose about 0.6 us each.
+template <typename Kernel, typename... Args>
+int launchDependent(Kernel kernel, unsigned ctas, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return TCPXB_K_OK;
+}
+
 template <int RED, bool L2RED, int FAN>
-int launch(const UnpackParams& p, int max_ctas, bool early, cudaStream_t stream) {
+int launch(const UnpackParams& p, int max_ctas, cudaStream_t stream) {
   using C = Cfg<RED, L2RED, FAN>;
   int dev = 0;
   int rc = deviceInfo(&dev);
@@ -796,22 +1092,20 @@ int launch(const UnpackParams& p, int max_ctas, bool early, cudaStream_t stream)
   rc = prepareVariant<RED, L2RED, FAN>(dev);
   if (rc) return rc;
   if (p.count == 0) return TCPXB_K_OK;
-  int ctas = (int)((p.count + kWarps - 1) / kWarps);
-  int cap = g_dev[dev].sms;
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
-  if (ctas > cap) ctas = cap;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = C::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = early ? 1 : 0;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, unpack_kernel<RED, L2RED, FAN>, p));
-  return TCPXB_K_OK;
+  const int sms = g_dev[dev].sms;
+  const bool whole_gpu = max_ctas <= 0 || max_ctas >= sms;
+  if constexpr (FAN == FAN_NONE && !L2RED) {
+    // Up to one record per ring warp the ring kernel is ahead (4 MiB in pages: 2.4 against 3.2 us, its bulk
+    // copies need one instruction per page); beyond that its second, part-filled round costs more than it saves.
+    // A launch confined to a few CTAs, streamed or asked to publish its completion stays with the ring.
+    if (whole_gpu && p.ready == nullptr && p.flag_value == 0 && p.count > (uint32_t)(sms * kWarps))
+      return launchDependent(unpack_wide_kernel<RED>, (p.count + kWideWarps - 1) / kWideWarps, kWideThreads, 0, stream, p);
+  }
+  // As many SMs as there are records before any SM gets a second one: a record is one warp's work, and 12 of
+  // them on one SM share its bulk-copy engine (256 records: 3.1 us on 22 SMs, 2.3 us on 148).
+  const int cap = whole_gpu ? sms : max_ctas;
+  const int ctas = p.count < (uint32_t)cap ? (int)p.count : cap;
+  return launchDependent(unpack_kernel<RED, L2RED, FAN>, (unsigned)ctas, kThreads, C::kSmemBytes, stream, p);
 }
 
 // Device address of the allocation-free checksum's scratch on `dev` (the current
@@ -841,16 +1135,16 @@ int prepareFan(int dev) {
 }
 
 template <int FAN>
-int dispatch(const UnpackParams& p, int dtype, int impl, int max_ctas, bool early, cudaStream_t s) {
+int dispatch(const UnpackParams& p, int dtype, int impl, int max_ctas, cudaStream_t s) {
   const bool l2 = (impl == TCPXB_REDUCE_L2);
   switch (dtype) {
-    case TCPXB_U8: return launch<TCPXB_U8, false, FAN>(p, max_ctas, early, s);
+    case TCPXB_U8: return launch<TCPXB_U8, false, FAN>(p, max_ctas, s);
     case TCPXB_BF16:
-      return l2 ? launch<TCPXB_BF16, true, FAN>(p, max_ctas, early, s)
-                : launch<TCPXB_BF16, false, FAN>(p, max_ctas, early, s);
+      return l2 ? launch<TCPXB_BF16, true, FAN>(p, max_ctas, s)
+                : launch<TCPXB_BF16, false, FAN>(p, max_ctas, s);
     case TCPXB_F32:
-      return l2 ? launch<TCPXB_F32, true, FAN>(p, max_ctas, early, s)
-                : launch<TCPXB_F32, false, FAN>(p, max_ctas, early, s);
+      return l2 ? launch<TCPXB_F32, true, FAN>(p, max_ctas, s)
+                : launch<TCPXB_F32, false, FAN>(p, max_ctas, s);
     default: return fail(TCPXB_K_INVALID, "unknown dtype");
   }
 }
@@ -929,6 +1223,9 @@ int tcpxb_kernels_preload(void) {
   TCPXB_DRY_FAN(FAN_PEER);
   TCPXB_DRY_FAN(FAN_NVLS);
 #undef TCPXB_DRY_FAN
+  unpack_wide_kernel<TCPXB_U8><<<1, kWideThreads, 0, s>>>(p);
+  unpack_wide_kernel<TCPXB_BF16><<<1, kWideThreads, 0, s>>>(p);
+  unpack_wide_kernel<TCPXB_F32><<<1, kWideThreads, 0, s>>>(p);
 #undef TCPXB_DRY
   wait_flags_kernel<<<1, 32, 0, s>>>(nullptr, 0, 0, 1, nullptr);
   SignalParams sp;
@@ -947,6 +1244,7 @@ int tcpxb_kernels_preload(void) {
   CUDA_TRY(cudaMemsetAsync(cs, 0, 8, s));
   checksum_kernel<<<1, kCsumThreads, 0, s>>>(nullptr, 0, &static_cast<CsumScratch*>(cs)->partial[kCsumBlocks - 1],
                                              static_cast<CsumScratch*>(cs));
+  stage_out_kernel<<<1, kStageThreads, 0, s>>>(nullptr, nullptr, 0, nullptr, &static_cast<CsumScratch*>(cs)->pad, 0);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(s));
   CUDA_TRY(cudaStreamDestroy(s));
@@ -961,7 +1259,7 @@ int tcpxb_unpack_copy(const void* pool, uint64_t pool_bytes, void* dst, uint64_t
   int rc = fill(p, pool, pool_bytes, nullptr, dst, nullptr, dst_bytes, nullptr, 0, descs, count,
                 status, opts);
   if (rc) return rc;
-  return dispatch<FAN_NONE>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0,
+  return dispatch<FAN_NONE>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -976,7 +1274,7 @@ int tcpxb_unpack_reduce(const void* pool, uint64_t pool_bytes, const void* acc, 
   int rc = fill(p, pool, pool_bytes, acc, dst, nullptr, dst_bytes, nullptr, 0, descs, count, status,
                 opts);
   if (rc) return rc;
-  return dispatch<FAN_NONE>(p, dtype, impl, opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0,
+  return dispatch<FAN_NONE>(p, dtype, impl, opts ? opts->max_ctas : 0,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -987,7 +1285,7 @@ int tcpxb_unpack_fanout(const void* pool, uint64_t pool_bytes, void* dst, uint64
   int rc = fill(p, pool, pool_bytes, nullptr, dst, nullptr, dst_bytes, peers, npeers, descs, count,
                 status, opts);
   if (rc) return rc;
-  return dispatch<FAN_PEER>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0,
+  return dispatch<FAN_PEER>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -1003,7 +1301,7 @@ int tcpxb_unpack_reduce_fanout(const void* pool, uint64_t pool_bytes, const void
   int rc = fill(p, pool, pool_bytes, acc, dst, nullptr, dst_bytes, peers, npeers, descs, count,
                 status, opts);
   if (rc) return rc;
-  return dispatch<FAN_PEER>(p, dtype, impl, opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0,
+  return dispatch<FAN_PEER>(p, dtype, impl, opts ? opts->max_ctas : 0,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -1016,7 +1314,7 @@ int tcpxb_unpack_fanout_nvls(const void* pool, uint64_t pool_bytes, void* dst, v
   int rc = fill(p, pool, pool_bytes, nullptr, dst, mc_dst, dst_bytes, peers, npeers, descs, count,
                 status, opts);
   if (rc) return rc;
-  return dispatch<FAN_NVLS>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0,
+  return dispatch<FAN_NVLS>(p, TCPXB_U8, 0, opts ? opts->max_ctas : 0,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -1034,17 +1332,15 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
   if (rc) return rc;
   // acc == NULL selects the reduce-into-all form (multimem.red into every accumulator).
   return dispatch<FAN_NVLS>(p, dtype, acc == nullptr ? TCPXB_REDUCE_L2 : TCPXB_REDUCE_SM,
-                            opts ? opts->max_ctas : 0, opts != nullptr && opts->early_launch != 0, static_cast<cudaStream_t>(stream));
+                            opts ? opts->max_ctas : 0, static_cast<cudaStream_t>(stream));
 }
 
 int tcpxb_wait_flags(const uint32_t* flags, int n, uint32_t value, uint64_t wait_ns,
                      uint32_t* status, void* stream) {
   if (flags == nullptr || n < 0 || n > 32) return fail(TCPXB_K_INVALID, "bad flag table");
   if (n == 0) return TCPXB_K_OK;
-  wait_flags_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      flags, n, value, wait_ns ? wait_ns : kDefaultWaitNs, status);
-  CUDA_TRY(cudaGetLastError());
-  return TCPXB_K_OK;
+  return launchDependent(wait_flags_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), flags, n, value,
+                         wait_ns ? wait_ns : kDefaultWaitNs, status);
 }
 
 int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void* stream) {
@@ -1056,9 +1352,17 @@ int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void*
   for (int i = 0; i < n; ++i) p.flags[i] = peer_flags[i];
   p.n = n;
   p.value = value;
-  signal_flags_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  CUDA_TRY(cudaGetLastError());
-  return TCPXB_K_OK;
+  return launchDependent(signal_flags_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), p);
+}
+
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value,
+                    void* stream) {
+  if (flag == nullptr || ticket == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
+    return fail(TCPXB_K_INVALID, "null source, destination, ticket or flag");
+  const uint64_t want = (bytes + kStageThreads * 16 - 1) / (kStageThreads * 16);
+  const unsigned blocks = (unsigned)(want < 1 ? 1 : want > 64 ? 64 : want);
+  return launchDependent(stage_out_kernel, blocks, kStageThreads, 0, static_cast<cudaStream_t>(stream),
+                         static_cast<const uint8_t*>(src), static_cast<uint8_t*>(host_dst), bytes, ticket, flag, value);
 }
 
 int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_off, uint64_t bytes,
@@ -1081,16 +1385,15 @@ int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_of
   p.shard_off = shard_off;
   p.vecs = bytes >> 4;
   if (p.vecs == 0) return TCPXB_K_OK;
-  int dev = 0, sms = 0;
-  CUDA_TRY(cudaGetDevice(&dev));
-  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int dev = 0;
+  const int rc = deviceInfo(&dev);
+  if (rc) return rc;
+  const int sms = g_dev[dev].sms;
   uint64_t want = (p.vecs + 255) / 256;
   int blocks = (int)(want < (uint64_t)sms * 8 ? want : (uint64_t)sms * 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == TCPXB_BF16) peer_reduce_kernel<TCPXB_BF16><<<blocks, 256, 0, s>>>(p);
-  else peer_reduce_kernel<TCPXB_F32><<<blocks, 256, 0, s>>>(p);
-  CUDA_TRY(cudaGetLastError());
-  return TCPXB_K_OK;
+  return launchDependent(dtype == TCPXB_BF16 ? peer_reduce_kernel<TCPXB_BF16> : peer_reduce_kernel<TCPXB_F32>, (unsigned)blocks, 256, 0,
+                         s, p);
 }
 
 size_t tcpxb_checksum_scratch_bytes(void) { return sizeof(CsumScratch); }
@@ -1102,10 +1405,8 @@ int tcpxb_checksum(const void* buf, uint64_t bytes, uint64_t* out, void* partial
     return fail(TCPXB_K_INVALID, "checksum buffer must be 4-byte aligned");
   uint64_t want = (bytes / 16 + kCsumThreads - 1) / kCsumThreads;
   int blocks = (int)(want < 1 ? 1 : (want > (uint64_t)kCsumBlocks ? kCsumBlocks : want));
-  checksum_kernel<<<blocks, kCsumThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint8_t*>(buf), bytes, out, static_cast<CsumScratch*>(partials));
-  CUDA_TRY(cudaGetLastError());
-  return TCPXB_K_OK;
+  return launchDependent(checksum_kernel, (unsigned)blocks, kCsumThreads, 0, static_cast<cudaStream_t>(stream),
+                         static_cast<const uint8_t*>(buf), bytes, out, static_cast<CsumScratch*>(partials));
 }
 
 int tcpxb_checksum_noalloc(const void* buf, uint64_t bytes, uint64_t* out, void* stream) {
@@ -1127,10 +1428,8 @@ int tcpxb_checksum_noalloc(const void* buf, uint64_t bytes, uint64_t* out, void*
   CUDA_TRY(cudaMemsetAsync(scratch, 0, 8, s));
   uint64_t want = (bytes / 16 + kCsumThreads - 1) / kCsumThreads;
   int blocks = (int)(want < 1 ? 1 : (want > (uint64_t)kCsumBlocks ? kCsumBlocks : want));
-  checksum_kernel<<<blocks, kCsumThreads, 0, s>>>(static_cast<const uint8_t*>(buf), bytes, out,
-                                                  static_cast<CsumScratch*>(scratch));
-  CUDA_TRY(cudaGetLastError());
-  return TCPXB_K_OK;
+  return launchDependent(checksum_kernel, (unsigned)blocks, kCsumThreads, 0, s, static_cast<const uint8_t*>(buf), bytes, out,
+                         static_cast<CsumScratch*>(scratch));
 }
 
 }  // extern "C"
