@@ -490,6 +490,7 @@ Result ensureTxStage(Comm* comm) {
   if (comm->tx_stage_bytes == 0) comm->tx_stage_bytes = (uint64_t)flags().tx_staging_bytes;
   TCPXB_CHECK(gpu::hostAllocMapped(comm->tx_stage_bytes, &h, &d));
   comm->tx_stage = static_cast<uint8_t*>(h);
+  comm->tx_stage_dev = static_cast<uint8_t*>(d);
   return kSuccess;
 }
 
@@ -519,6 +520,19 @@ Result startCudaSend(Comm* comm, Request* r, MemHandle* mh) {
     return kInvalidArgument;
   }
   if (!stageAlloc(comm, (uint64_t)r->size, &r->stage, &r->stage_bytes)) return kInProgress;
+  if (comm->send_on_caller) {
+    // One launch instead of an event record, a stream wait, a copy and a counter write, and no hop between streams.
+    r->seg_bytes = r->size;
+    r->n_segs = 1;
+    r->segs_done = 0;
+    uint32_t* flag = comm->stage_marks.take(&r->seg_mark[0]);
+    if (tcpxb_stage_out(r->data, comm->tx_stage_dev + (r->stage - comm->tx_stage), (uint64_t)r->size, flag, r->seg_mark[0],
+                        comm->send_stream) != 0) {
+      WARN("staging launch failed: %s", tcpxb_kernel_last_error());
+      return kUnhandledCudaError;
+    }
+    return kSuccess;
+  }
   // One staging copy per ~2 MiB: enough to let the first chunks leave while the
   // rest is still being copied, few enough that the per-copy launch cost stays small.
   const int chunk = chunkBytesFor(r->size, comm->num_socks);
@@ -1376,7 +1390,15 @@ Result netIrecvConsumed(Comm* comm, int n, Request* r) {
   return kSuccess;
 }
 
-void netSetSendDependency(Comm* comm, gpu::Event event) { comm->send_dependency = event; }
+void netSetSendDependency(Comm* comm, gpu::Event event) {
+  comm->send_dependency = event;
+  comm->send_on_caller = false;
+}
+void netSetSendStream(Comm* comm, gpu::Stream stream) {
+  comm->send_on_caller = true;
+  comm->send_stream = stream;
+  comm->send_dependency = nullptr;
+}
 
 void netSetHelperNap(Comm* comm, int nap_us, int rounds) {
   if (comm == nullptr) return;

@@ -148,6 +148,10 @@ struct Engine {
 };
 
 constexpr double kSmallExchangeSpinUs = 250.0;
+constexpr double kLastKernelSpinUs = 200.0;
+// Up to here a whole exchange is staged by kernels on the caller's stream, where they queue before its unpack kernels.
+// Larger ones overlap staging with unpacking, which needs a stream of its own, and the copy engine takes no SM for it.
+constexpr uint64_t kStageKernelBytes = 64 << 10;
 
 // One look at every receive comm's control socket: a single poll() with no wait, then a
 // hint to the comms whose socket has data.  Replaces one recv() attempt per comm and
@@ -216,9 +220,10 @@ int checkDeviceStatus(Engine* e) {
   return -1;
 }
 
-// Launches the unpack kernel for one finished receive request.
+// Launches the unpack kernel for one finished receive request; `*done_mark` is the value that
+// e->kernel_marks reaches once it has finished.
 int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_off, uint64_t len, bool publish,
-                 void* stream) {
+                 void* stream, uint32_t* done_mark) {
   ScatterList sl;
   ENG_NET(netRequestScatterList(req, &sl));
   e->stats.fragments += sl.count;
@@ -230,6 +235,7 @@ int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_of
   const uint8_t* acc = rs.acc ? rs.acc + region_off : nullptr;
   const tcpxbLoadMeta* descs = reinterpret_cast<const tcpxbLoadMeta*>(sl.dev);
   const uint32_t count = (uint32_t)sl.count;
+  if (count == 0) return fail("a finished receive without fragments%s", "");
   void* peers[TCPXB_MAX_PEERS];
   int npeers = 0;
   const bool fan = rs.fanout && e->G > 1;
@@ -242,7 +248,6 @@ int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_of
     }
     if (publish) {
       opts.flag_value = e->epoch;
-      opts.ticket = e->ticket;
     }
   }
   if (e->cfg.plain_mode) {
@@ -269,27 +274,17 @@ int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_of
       for (int i = 0; i < npeers; ++i) pf[i] = opts.peer_flags[i];
       ENG_K(tcpxb_signal_flags(pf, npeers, e->epoch, stream));
     }
+    ENG_NET(e->kernel_marks.mark(stream, done_mark));
     return 0;
   }
+  // The kernel advances the counter itself: a stream memory operation behind it would be a second driver call
+  // per request and one more step between the kernel's last store and the host.
+  opts.ticket = e->ticket;
+  uint32_t* done = e->kernel_marks.take(done_mark);
   const bool nvls = fan && e->cfg.use_nvls && e->mc_out != nullptr;
-  if (acc == nullptr) {
-    if (!fan) ENG_K(tcpxb_unpack_copy(sl.pool_dev, sl.pool_bytes, dst, len, descs, count, e->status_dev, &opts, stream));
-    else if (nvls)
-      ENG_K(tcpxb_unpack_fanout_nvls(sl.pool_dev, sl.pool_bytes, dst, e->mc_out + rs.out_offset + region_off, len, peers,
-                                     npeers, descs, count, e->status_dev, &opts, stream));
-    else
-      ENG_K(tcpxb_unpack_fanout(sl.pool_dev, sl.pool_bytes, dst, len, peers, npeers, descs, count, e->status_dev, &opts, stream));
-  } else {
-    if (!fan)
-      ENG_K(tcpxb_unpack_reduce(sl.pool_dev, sl.pool_bytes, acc, dst, len, descs, count, rs.dtype,
-                                acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM, e->status_dev, &opts, stream));
-    else if (nvls)
-      ENG_K(tcpxb_unpack_reduce_fanout_nvls(sl.pool_dev, sl.pool_bytes, acc, dst, e->mc_out + rs.out_offset + region_off, len,
-                                            peers, npeers, descs, count, rs.dtype, e->status_dev, &opts, stream));
-    else
-      ENG_K(tcpxb_unpack_reduce_fanout(sl.pool_dev, sl.pool_bytes, acc, dst, len, peers, npeers, descs, count, rs.dtype,
-                                       TCPXB_REDUCE_SM, e->status_dev, &opts, stream));
-  }
+  ENG_K(tcpxb_unpack_request(sl.pool_dev, sl.pool_bytes, acc, dst, nvls ? e->mc_out + rs.out_offset + region_off : nullptr, len, peers,
+                             npeers, descs, count, rs.dtype, !fan && acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM, e->status_dev,
+                             &opts, done, *done_mark, stream));
   return 0;
 }
 
@@ -307,8 +302,12 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
   std::vector<std::deque<PendingUnpack>> uq(R);
   if (ss.bytes > 0) {
     // sends may read only what the stream has produced so far
-    ENG_NET(gpu::eventRecord(e->dep_event, stream));
-    for (int r = 0; r < R; ++r) netSetSendDependency(e->rails[r].send, e->dep_event);
+    if (ss.bytes <= kStageKernelBytes && (reinterpret_cast<uintptr_t>(ss.src) & 15) == 0) {
+      for (int r = 0; r < R; ++r) netSetSendStream(e->rails[r].send, stream);
+    } else {
+      ENG_NET(gpu::eventRecord(e->dep_event, stream));
+      for (int r = 0; r < R; ++r) netSetSendDependency(e->rails[r].send, e->dep_event);
+    }
   }
   MemHandle send_mh{const_cast<uint8_t*>(ss.src), ss.bytes, kPtrCuda, e->cfg.gpu_dev};
   MemHandle recv_mh{rs.dst, rs.bytes, kPtrCuda, e->cfg.gpu_dev};
@@ -373,9 +372,8 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
         // one that publishes completion.
         const bool publish = rs.last && (launched_r + 1 == n_recv);
         lap(e->stats.t_test_recv);
-        ENG_TRY(launchUnpack(e, rq[r].front(), rs, off, want, publish, stream));
         uint32_t done_mark = 0;
-        ENG_NET(e->kernel_marks.mark(stream, &done_mark));
+        ENG_TRY(launchUnpack(e, rq[r].front(), rs, off, want, publish, stream, &done_mark));
         uq[r].push_back({rq[r].front(), done_mark});
         rq[r].pop_front();
         rq_idx[r].pop_front();
@@ -444,7 +442,14 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
   // pool pages go back once the kernels that read them have finished
   bool any_left = false;
   for (int r = 0; r < R; ++r) any_left = any_left || !uq[r].empty();
-  if (any_left) ENG_NET(gpu::streamSynchronize(stream));
+  if (any_left) {
+    // The last kernels end within tens of microseconds, and their counter says so sooner than a stream
+    // synchronise returns.  A kernel that failed never writes it: the stream has the reason.
+    const uint32_t last = e->kernel_marks.issued();
+    const double t1 = nowSec();
+    while (!e->kernel_marks.reached(last) && (nowSec() - t1) * 1e6 < kLastKernelSpinUs) __builtin_ia32_pause();
+    if (!e->kernel_marks.reached(last)) ENG_NET(gpu::streamSynchronize(stream));
+  }
   for (int r = 0; r < R; ++r) {
     while (!uq[r].empty()) {
       if (!e->kernel_marks.reached(uq[r].front().mark)) return fail("unpack completion mark missing after a stream synchronize%s", "");

@@ -86,6 +86,8 @@ class StreamCounter {
   bool ready() const { return host_ != nullptr; }
   // Queues the next value on `s` and returns it in *value.
   Result mark(Stream s, uint32_t* value);
+  // The next value and the device address of the counter, for a kernel that writes it itself at its end.
+  uint32_t* take(uint32_t* value) { *value = ++issued_; return dev_; }
   bool reached(uint32_t value) const { return (int32_t)(__atomic_load_n(host_, __ATOMIC_ACQUIRE) - value) >= 0; }
   uint32_t issued() const { return issued_; }
 

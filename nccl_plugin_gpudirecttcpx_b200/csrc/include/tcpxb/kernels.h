@@ -129,6 +129,17 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
                                     uint32_t count, int dtype, uint32_t* status,
                                     const tcpxbUnpackOpts* opts, void* stream);
 
+// Any of the above for a host that polls for the end of the launch: a copy when acc is NULL, else a
+// reduce (impl as for K2); the fan-out to `peers` when npeers > 0, through mc_dst when that is not
+// NULL.  The launch ends with *done_flag = done_value (release, system scope; mapped host memory),
+// errors or not, once every store of the launch is visible and every byte of the pool has been read.
+// opts->ticket is required.  An empty list launches nothing and writes nothing.
+int tcpxb_unpack_request(const void* pool, uint64_t pool_bytes, const void* acc, void* dst,
+                         void* mc_dst, uint64_t dst_bytes, void* const* peers, int npeers,
+                         const tcpxbLoadMeta* descs, uint32_t count, int dtype, int impl,
+                         uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag,
+                         uint32_t done_value, void* stream);
+
 // Loads every kernel of this library on the current device and applies their
 // launch attributes.  CUDA loads kernels lazily, and a first launch may have to
 // wait for running kernels to finish; a receive path that launches its first
@@ -147,10 +158,9 @@ int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void*
 
 // Copies `bytes` from device memory to mapped host memory and then writes `value` to
 // *flag (release, system scope; mapped host memory too): a small message's way to its
-// staging buffer, in stream order and without the copy engine.  `ticket` is one
-// zero-initialised uint32 on the launching GPU; the kernel leaves it zero.
-int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket,
-                    uint32_t* flag, uint32_t value, void* stream);
+// staging buffer, in stream order and without the copy engine.
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* flag,
+                    uint32_t value, void* stream);
 
 // Intra-node reduce-scatter stage over peer memory: out[i] = sum over r of
 // srcs[r][shard_off + i], element-wise, for `bytes` bytes.  srcs are peer-mapped

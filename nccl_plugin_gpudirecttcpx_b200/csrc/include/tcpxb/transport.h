@@ -247,10 +247,13 @@ struct Comm {
   RxBufMgr* rxmgr = nullptr;
   std::unique_ptr<DevQueue> devq;
   uint8_t* tx_stage = nullptr;
+  uint8_t* tx_stage_dev = nullptr;  // the same memory as the GPU addresses it
   uint64_t tx_stage_bytes = 0, tx_head = 0, tx_tail = 0;  // ring offsets (monotonic)
   uint32_t* unpack_status_host = nullptr;
   uint32_t* unpack_status_dev = nullptr;
   gpu::Event send_dependency = nullptr;
+  bool send_on_caller = false;  // staging runs as a kernel on send_stream, not on the copy engine behind send_dependency
+  gpu::Stream send_stream = nullptr;
   // stream-ordered completion counters in mapped host memory: staging copies (send
   // side) and unpack kernels / page placements (receive side) on `stream`
   gpu::StreamCounter stage_marks, unpack_marks;
@@ -346,6 +349,9 @@ constexpr int kMaxAdaptiveChunk = 4 << 20;
 // The next netIsend of a CUDA buffer on `comm` first makes the comm's copy stream
 // wait for `event` (the kernel that produces the data), then stages the data.
 void netSetSendDependency(Comm* comm, gpu::Event event);
+// Until the next netSetSendDependency: device-memory sends are staged by a kernel on `stream`, behind what it
+// holds, instead of by the copy engine on the comm's own stream.  For small messages; all earlier sends must be done.
+void netSetSendStream(Comm* comm, gpu::Stream stream);
 
 // Scatter list of a finished unpack-mode receive.
 struct ScatterList {

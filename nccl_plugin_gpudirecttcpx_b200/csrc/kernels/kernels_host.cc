@@ -225,6 +225,25 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
                                     status, opts, stream);
 }
 
+int tcpxb_unpack_request(const void* pool, uint64_t pool_bytes, const void* acc, void* dst, void* mc_dst, uint64_t dst_bytes,
+                         void* const* peers, int npeers, const tcpxbLoadMeta* descs, uint32_t count, int dtype, int impl,
+                         uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag, uint32_t done_value, void* stream) {
+  if (done_flag == nullptr || opts == nullptr || opts->ticket == nullptr) return fail(TCPXB_K_INVALID, "a completion word and its ticket are needed");
+  int rc;
+  if (mc_dst != nullptr && acc != nullptr)
+    rc = tcpxb_unpack_reduce_fanout_nvls(pool, pool_bytes, acc, dst, mc_dst, dst_bytes, peers, npeers, descs, count, dtype, status, opts, stream);
+  else if (mc_dst != nullptr)
+    rc = tcpxb_unpack_fanout_nvls(pool, pool_bytes, dst, mc_dst, dst_bytes, peers, npeers, descs, count, status, opts, stream);
+  else if (acc == nullptr)
+    rc = tcpxb_unpack_fanout(pool, pool_bytes, dst, dst_bytes, peers, npeers, descs, count, status, opts, stream);
+  else if (npeers > 0)
+    rc = tcpxb_unpack_reduce_fanout(pool, pool_bytes, acc, dst, dst_bytes, peers, npeers, descs, count, dtype, impl, status, opts, stream);
+  else
+    rc = tcpxb_unpack_reduce(pool, pool_bytes, acc, dst, dst_bytes, descs, count, dtype, impl, status, opts, stream);
+  if (rc == TCPXB_K_OK && count != 0) __atomic_store_n(done_flag, done_value, __ATOMIC_RELEASE);
+  return rc;
+}
+
 int tcpxb_wait_flags(const uint32_t* flags, int n, uint32_t value, uint64_t wait_ns, uint32_t* status, void*) {
   if (flags == nullptr || n < 0) return fail(TCPXB_K_INVALID, "null flag array");
   const uint64_t limit = wait_ns ? wait_ns : kDefaultWaitNs;
@@ -246,9 +265,9 @@ int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void*
   return TCPXB_K_OK;
 }
 
-int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value, void*) {
-  if (flag == nullptr || ticket == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
-    return fail(TCPXB_K_INVALID, "null source, destination, ticket or flag");
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* flag, uint32_t value, void*) {
+  if (flag == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
+    return fail(TCPXB_K_INVALID, "null source, destination or flag");
   if (tcpxb::gpu::standinMovesData()) memcpy(host_dst, src, bytes);
   __atomic_store_n(flag, value, __ATOMIC_RELEASE);
   return TCPXB_K_OK;

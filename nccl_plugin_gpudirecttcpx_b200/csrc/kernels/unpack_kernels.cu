@@ -72,6 +72,8 @@ struct UnpackParams {
   uint32_t* peer_flags[TCPXB_MAX_PEERS];
   uint32_t flag_value;
   uint32_t* ticket;
+  uint32_t* done_flag;
+  uint32_t done_value;
   uint32_t* status;
   const uint32_t* ready;
   uint64_t wait_ns;
@@ -662,9 +664,9 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
   }
   if (lane == 0) bulk_wait_all();
 
-  if (p.flag_value != 0 && p.ticket != nullptr) {
-    // Publish completion (to the peers, or to a host that watches a mapped word) once every
-    // CTA's stores are done.
+  if ((p.flag_value != 0 || p.done_flag != nullptr) && p.ticket != nullptr) {
+    // Publish completion once every CTA's stores are done: to the peers (unless there were errors), and to
+    // a host that watches a mapped word.
     // The ticket counts CTAs in its low half and CTAs with errors in its high half.
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -674,11 +676,12 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
       if ((t & 0xffffu) == gridDim.x) {
         *p.ticket = 0;
         __threadfence_system();
-        if ((t >> 16) == 0) {
+        if (p.flag_value != 0 && (t >> 16) == 0) {
           for (int r = 0; r < TCPXB_MAX_PEERS; ++r) {
             if (p.peer_flags[r] != nullptr) st_release_sys(p.peer_flags[r], p.flag_value);
           }
         }
+        if (p.done_flag != nullptr) st_release_sys(p.done_flag, p.done_value);
       }
     }
   }
@@ -851,26 +854,23 @@ __global__ void signal_flags_kernel(const __grid_constant__ SignalParams p) {
   }
 }
 
-// Device memory -> mapped host memory, then a flag.  Bound by the PCIe write latency at these sizes
-// (up to 64 KiB): 4 KiB per CTA, one 16-byte vector per thread, all of them posted at once.
-constexpr int kStageThreads = 256;
+// Device memory -> mapped host memory, then a flag.  Bound by the latency of the launch and of one PCIe write:
+// one CTA moves all of it (up to 64 KiB in the engine), so that the flag needs no counting of CTAs.  Against the
+// copy engine behind an event, with a stream memory operation as the flag, and the same for the unpack kernel's
+// end: an all_reduce of 1 KiB 53 -> 49 us, of 64 KiB 66 -> 60 us.
+constexpr int kStageThreads = 1024;
 __global__ void __launch_bounds__(kStageThreads)
-stage_out_kernel(const uint8_t* src, uint8_t* dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value) {
-  const uint64_t stride = (uint64_t)gridDim.x * kStageThreads;
-  const uint64_t tid = (uint64_t)blockIdx.x * kStageThreads + threadIdx.x;
+stage_out_kernel(const uint8_t* src, uint8_t* dst, uint64_t bytes, uint32_t* flag, uint32_t value) {
   const uint64_t vecs = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? bytes >> 4 : 0;
   pdl_launch_dependents();
   pdl_wait();
-  for (uint64_t i = tid; i < vecs; i += stride) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
-  for (uint64_t i = (vecs << 4) + tid; i < bytes; i += stride) dst[i] = src[i];
+#pragma unroll 4
+  for (uint64_t i = threadIdx.x; i < vecs; i += blockDim.x) *reinterpret_cast<uint4*>(dst + (i << 4)) = ld_v4(src + (i << 4));
+  for (uint64_t i = (vecs << 4) + threadIdx.x; i < bytes; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence_system();
-    if (gridDim.x == 1 || atomicAdd(ticket, 1u) == gridDim.x - 1) {
-      if (gridDim.x != 1) *ticket = 0;
-      __threadfence_system();
-      st_release_sys(flag, value);
-    }
+    st_release_sys(flag, value);
   }
 }
 
@@ -1098,7 +1098,7 @@ int launch(const UnpackParams& p, int max_ctas, cudaStream_t stream) {
     // Up to one record per ring warp the ring kernel is ahead (4 MiB in pages: 2.4 against 3.2 us, its bulk
     // copies need one instruction per page); beyond that its second, part-filled round costs more than it saves.
     // A launch confined to a few CTAs, streamed or asked to publish its completion stays with the ring.
-    if (whole_gpu && p.ready == nullptr && p.flag_value == 0 && p.count > (uint32_t)(sms * kWarps))
+    if (whole_gpu && p.ready == nullptr && p.flag_value == 0 && p.done_flag == nullptr && p.count > (uint32_t)(sms * kWarps))
       return launchDependent(unpack_wide_kernel<RED>, (p.count + kWideWarps - 1) / kWideWarps, kWideThreads, 0, stream, p);
   }
   // As many SMs as there are records before any SM gets a second one: a record is one warp's work, and 12 of
@@ -1244,7 +1244,7 @@ int tcpxb_kernels_preload(void) {
   CUDA_TRY(cudaMemsetAsync(cs, 0, 8, s));
   checksum_kernel<<<1, kCsumThreads, 0, s>>>(nullptr, 0, &static_cast<CsumScratch*>(cs)->partial[kCsumBlocks - 1],
                                              static_cast<CsumScratch*>(cs));
-  stage_out_kernel<<<1, kStageThreads, 0, s>>>(nullptr, nullptr, 0, nullptr, &static_cast<CsumScratch*>(cs)->pad, 0);
+  stage_out_kernel<<<1, kStageThreads, 0, s>>>(nullptr, nullptr, 0, &static_cast<CsumScratch*>(cs)->pad, 0);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(s));
   CUDA_TRY(cudaStreamDestroy(s));
@@ -1335,6 +1335,27 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
                             opts ? opts->max_ctas : 0, static_cast<cudaStream_t>(stream));
 }
 
+int tcpxb_unpack_request(const void* pool, uint64_t pool_bytes, const void* acc, void* dst, void* mc_dst, uint64_t dst_bytes,
+                         void* const* peers, int npeers, const tcpxbLoadMeta* descs, uint32_t count, int dtype, int impl,
+                         uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag, uint32_t done_value, void* stream) {
+  if (done_flag == nullptr || opts == nullptr || opts->ticket == nullptr)
+    return fail(TCPXB_K_INVALID, "a completion word and its ticket are needed");
+  if (acc != nullptr && dtype != TCPXB_BF16 && dtype != TCPXB_F32)
+    return fail(TCPXB_K_INVALID, "reduce needs dtype bf16 or f32");
+  if (impl == TCPXB_REDUCE_L2 && acc != nullptr && (acc != dst || mc_dst != nullptr))
+    return fail(TCPXB_K_INVALID, "the L2 reduce form is in place: acc must be dst");
+  UnpackParams p;
+  int rc = fill(p, pool, pool_bytes, acc, dst, mc_dst, dst_bytes, peers, npeers, descs, count, status, opts);
+  if (rc) return rc;
+  p.done_flag = done_flag;
+  p.done_value = done_value;
+  const int dt = acc != nullptr ? dtype : TCPXB_U8;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (mc_dst != nullptr) return dispatch<FAN_NVLS>(p, dt, TCPXB_REDUCE_SM, opts->max_ctas, s);
+  if (npeers > 0) return dispatch<FAN_PEER>(p, dt, impl, opts->max_ctas, s);
+  return dispatch<FAN_NONE>(p, dt, impl, opts->max_ctas, s);
+}
+
 int tcpxb_wait_flags(const uint32_t* flags, int n, uint32_t value, uint64_t wait_ns,
                      uint32_t* status, void* stream) {
   if (flags == nullptr || n < 0 || n > 32) return fail(TCPXB_K_INVALID, "bad flag table");
@@ -1355,14 +1376,12 @@ int tcpxb_signal_flags(uint32_t* const* peer_flags, int n, uint32_t value, void*
   return launchDependent(signal_flags_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), p);
 }
 
-int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* ticket, uint32_t* flag, uint32_t value,
-                    void* stream) {
-  if (flag == nullptr || ticket == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
-    return fail(TCPXB_K_INVALID, "null source, destination, ticket or flag");
-  const uint64_t want = (bytes + kStageThreads * 16 - 1) / (kStageThreads * 16);
-  const unsigned blocks = (unsigned)(want < 1 ? 1 : want > 64 ? 64 : want);
-  return launchDependent(stage_out_kernel, blocks, kStageThreads, 0, static_cast<cudaStream_t>(stream),
-                         static_cast<const uint8_t*>(src), static_cast<uint8_t*>(host_dst), bytes, ticket, flag, value);
+int tcpxb_stage_out(const void* src, void* host_dst, uint64_t bytes, uint32_t* flag, uint32_t value, void* stream) {
+  if (flag == nullptr || (bytes != 0 && (src == nullptr || host_dst == nullptr)))
+    return fail(TCPXB_K_INVALID, "null source, destination or flag");
+  const unsigned threads = bytes <= kStageThreads * 16 / 4 ? kStageThreads / 4 : kStageThreads;
+  return launchDependent(stage_out_kernel, 1, threads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(src),
+                         static_cast<uint8_t*>(host_dst), bytes, flag, value);
 }
 
 int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_off, uint64_t bytes,
