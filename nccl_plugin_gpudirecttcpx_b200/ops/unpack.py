@@ -68,7 +68,7 @@ def _check(rc: int) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # without building a Stream object
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
