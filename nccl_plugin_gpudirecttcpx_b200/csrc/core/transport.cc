@@ -535,7 +535,7 @@ Result startCudaSend(Comm* comm, Request* r, MemHandle* mh) {
   }
   // One staging copy per ~2 MiB: enough to let the first chunks leave while the
   // rest is still being copied, few enough that the per-copy launch cost stays small.
-  const int chunk = chunkBytesFor(r->size, comm->num_socks);
+  const int chunk = chunkBytesFor(r->size, comm->num_socks, comm->least_chunk);
   int n_want = std::max(1, std::min(kMaxTxSegments, r->size / (2 << 20)));
   int seg = (r->size + n_want - 1) / n_want;
   seg = (seg + chunk - 1) / chunk * chunk;
@@ -728,13 +728,15 @@ Result launchUnpack(Comm* comm, Request* r) {
 // ADAPTIVE_CHUNK (default) a message is cut into about one chunk per socket instead:
 // the quantum grows to size / sockets, rounded up to a whole rx page, but never
 // beyond kMaxAdaptiveChunk, so that large messages still pipeline through the task rings.
-int chunkBytesFor(int message_bytes, int num_socks) {
+// A caller may lower the quantum to `least` for its own comms (netSetLeastChunk), so that a
+// message of a few quanta occupies every socket.
+int chunkBytesFor(int message_bytes, int num_socks, int64_t least) {
   const Flags& f = flags();
   int64_t chunk = f.dynamic_chunk_size;
   if (f.adaptive_chunk != 0 && num_socks > 0) {
     int64_t per_sock = ((int64_t)message_bytes + num_socks - 1) / num_socks;
     per_sock = (per_sock + kRxPageBytes - 1) / kRxPageBytes * kRxPageBytes;
-    chunk = std::max(chunk, std::min<int64_t>(per_sock, std::max<int64_t>(kMaxAdaptiveChunk, chunk)));
+    chunk = std::max(std::min(chunk, least), std::min<int64_t>(per_sock, std::max<int64_t>(kMaxAdaptiveChunk, chunk)));
   }
   return (int)std::min<int64_t>(chunk, INT32_MAX);
 }
@@ -770,7 +772,7 @@ Result progressSendRequest(Comm* comm, Request* r) {
     comm->rq.advance(kReqActive);
     return kSuccess;
   }
-  const int chunk_size = chunkBytesFor(r->size, comm->num_socks);
+  const int chunk_size = chunkBytesFor(r->size, comm->num_socks, comm->least_chunk);
   while (r->offset < r->size && comm->mapper->hasFlow()) {
     const int chunk = std::min(chunk_size, r->size - r->offset);
     // A chunk of a CUDA send is announced and queued before its staging copy has
@@ -1390,6 +1392,7 @@ Result netIrecvConsumed(Comm* comm, int n, Request* r) {
   return kSuccess;
 }
 
+void netSetLeastChunk(Comm* comm, int64_t bytes) { comm->least_chunk = bytes; }
 void netSetSendDependency(Comm* comm, gpu::Event event) {
   comm->send_dependency = event;
   comm->send_on_caller = false;

@@ -216,6 +216,7 @@ struct Comm {
   std::atomic<int> error{kSuccess};  // first fatal Result seen by any thread
   int dev = 0;
   int num_socks = 0, num_threads = 0;
+  int64_t least_chunk = INT64_MAX;  // see netSetLeastChunk
   SocketCtx sock[kMaxSockets];
   int ctrl_fd = -1;
   std::string ctrl_flow;
@@ -343,7 +344,9 @@ int netCtrlPollFd(Comm* comm);
 // paying a system call, on every progress round.
 void netHintCtrlReadable(Comm* comm);
 // Bytes per chunk for a message of `message_bytes` on a comm with `num_socks` data sockets.
-int chunkBytesFor(int message_bytes, int num_socks);
+int chunkBytesFor(int message_bytes, int num_socks, int64_t least = INT64_MAX);
+// With ADAPTIVE_CHUNK, messages of this send comm are cut down to `bytes` where NCCL_DYNAMIC_CHUNK_SIZE is larger.
+void netSetLeastChunk(Comm* comm, int64_t bytes);
 constexpr int kMaxAdaptiveChunk = 4 << 20;
 
 // The next netIsend of a CUDA buffer on `comm` first makes the comm's copy stream

@@ -1133,6 +1133,15 @@ TEST(chunk_size_follows_the_sockets) {
   EXPECT(chunkBytesFor(100000, 4) == 131072);           // small messages: one chunk of at most the quantum
   EXPECT(chunkBytesFor(64 << 20, 2) == kMaxAdaptiveChunk);
   EXPECT(chunkBytesFor(0, 4) == 131072);
+  // a caller that lowers the quantum for its own comms
+  setenv("NCCL_DYNAMIC_CHUNK_SIZE", "524288", 1);
+  reloadFlags();
+  EXPECT(chunkBytesFor(1 << 20, 4) == 524288);
+  EXPECT(chunkBytesFor(1 << 20, 4, 131072) == 262144);
+  EXPECT(chunkBytesFor(200000, 4, 131072) == 131072);
+  EXPECT(chunkBytesFor(8 << 20, 4, 131072) == 2 << 20);
+  EXPECT(chunkBytesFor(8 << 20, 4, 1 << 20) == 2 << 20);
+  setenv("NCCL_DYNAMIC_CHUNK_SIZE", "131072", 1);
   setenv("NCCL_GPUDIRECTTCPX_ADAPTIVE_CHUNK", "0", 1);
   reloadFlags();
   EXPECT(chunkBytesFor(4 << 20, 1) == 131072);
