@@ -133,6 +133,7 @@ struct Engine {
   tcpxbEngineStats stats;
   int req_bytes = 1 << 20, inflight = 4, ctas = 16;
   bool yield_when_idle = false;
+  bool ragged = false;  // see tcpxb_engine_set_ragged
   // idle policy of the driving thread
   Notifier notifier;
   int idle_spin_us = 20, idle_sleep_us = 30;
@@ -481,6 +482,8 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
   return 0;
 }
 
+uint64_t elementBytes(int dtype) { return dtype == TCPXB_BF16 ? 2 : 4; }
+
 int checkReady(Engine* e) {
   if (e == nullptr) return fail("null engine%s", "");
   if (!e->connected) return fail("engine is not connected%s", "");
@@ -722,7 +725,7 @@ int tcpxb_engine_all_reduce(void* engine, const void* in_, void* out_, uint64_t 
   Engine* e = static_cast<Engine*>(engine);
   ENG_TRY(checkReady(e));
   if (dtype != TCPXB_BF16 && dtype != TCPXB_F32) return fail("all_reduce needs bf16 or f32%s", "");
-  const uint64_t unit = (uint64_t)e->G * (uint64_t)(e->nodes > 2 ? e->nodes : 1) * 16;
+  const uint64_t unit = e->ragged && e->nodes == 2 ? elementBytes(dtype) : (uint64_t)e->G * (uint64_t)(e->nodes > 2 ? e->nodes : 1) * 16;
   if (bytes == 0 || bytes % unit != 0) return fail("all_reduce size must be a multiple of %s%ld bytes", "", (long)unit);
   const uint8_t* in = static_cast<const uint8_t*>(in_);
   uint8_t* out = static_cast<uint8_t*>(out_);
@@ -815,7 +818,7 @@ int tcpxb_engine_all_gather(void* engine, const void* in_, void* out_, uint64_t 
   Range range("tcpxb all_gather");
   Engine* e = static_cast<Engine*>(engine);
   ENG_TRY(checkReady(e));
-  if (B == 0 || B % 16 != 0) return fail("all_gather block must be a multiple of 16 bytes%s", "");
+  if (B == 0 || (B % 16 != 0 && !e->ragged)) return fail("all_gather block must be a multiple of 16 bytes%s", "");
   uint8_t* out = static_cast<uint8_t*>(out_);
   const int world_blocks = e->nodes * e->G;
   if (e->G > 1 && (out != e->out[e->local] || B * (uint64_t)world_blocks > e->buffer_bytes))
@@ -848,7 +851,7 @@ int tcpxb_engine_reduce_scatter(void* engine, const void* in_, void* out_, uint6
   Engine* e = static_cast<Engine*>(engine);
   ENG_TRY(checkReady(e));
   if (dtype != TCPXB_BF16 && dtype != TCPXB_F32) return fail("reduce_scatter needs bf16 or f32%s", "");
-  if (B == 0 || B % 16 != 0) return fail("reduce_scatter block must be a multiple of 16 bytes%s", "");
+  if (B == 0 || B % (e->ragged ? elementBytes(dtype) : 16) != 0) return fail("reduce_scatter block must be a multiple of 16 bytes%s", "");
   const uint8_t* in = static_cast<const uint8_t*>(in_);
   uint8_t* out = static_cast<uint8_t*>(out_);
   const int N = e->nodes;
@@ -856,6 +859,16 @@ int tcpxb_engine_reduce_scatter(void* engine, const void* in_, void* out_, uint6
     return fail("with several GPUs per node, in must be the registered work buffer%s", "");
   ++e->epoch;
   // 1. per node-block j: sum over the local GPUs of block (j, local) -> tmp[j]
+  auto mod = [N](int x) { return ((x % N) + N) % N; };
+  const bool apart = out + B <= in || in + B * (uint64_t)(e->twin ? 1 : N) <= out;
+  if (N == 2 && e->G == 1 && !e->cfg.plain_mode && apart) {
+    // One step: no running sum is written but the result, so both blocks are read where they are.
+    const int sp = mod(e->node - 1), rp = mod(e->node - 2);
+    SendSpec ss{B, in + (uint64_t)(e->twin ? 0 : sp) * B};
+    RecvSpec rs;
+    rs.bytes = B; rs.dtype = dtype; rs.acc = in + (uint64_t)(e->twin ? 0 : rp) * B; rs.dst = out;
+    return exchange(e, ss, rs, stream);
+  }
   ENG_TRY(ensureScratch(e, (uint64_t)N * B + (uint64_t)e->req_bytes));
   uint8_t* tmp = e->scratch;
   if (e->G > 1) {
@@ -871,7 +884,6 @@ int tcpxb_engine_reduce_scatter(void* engine, const void* in_, void* out_, uint6
     }
   }
   // 2. ring reduce-scatter over the nodes; the last step writes the result
-  auto mod = [N](int x) { return ((x % N) + N) % N; };
   for (int s = 0; s < N - 1; ++s) {
     const int sp = mod(e->node - s - 1), rp = mod(e->node - s - 2);
     SendSpec ss{B, tmp + (uint64_t)(e->twin ? rp : sp) * B};
@@ -888,6 +900,13 @@ int tcpxb_engine_reduce_scatter(void* engine, const void* in_, void* out_, uint6
     ENG_K(tcpxb_signal_flags(pf, n, e->epoch, stream));
     ENG_K(tcpxb_wait_flags(e->flags[e->local] + 32, e->G, e->epoch, 0, e->status_dev, stream));
   }
+  return 0;
+}
+
+int tcpxb_engine_set_ragged(void* engine, int on) {
+  Engine* e = static_cast<Engine*>(engine);
+  if (e == nullptr) return fail("null engine%s", "");
+  e->ragged = on != 0 && e->G == 1 && !e->cfg.plain_mode;
   return 0;
 }
 

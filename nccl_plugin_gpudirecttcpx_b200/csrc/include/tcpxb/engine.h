@@ -98,6 +98,10 @@ int tcpxb_engine_all_reduce(void* engine, const void* in, void* out, uint64_t by
 int tcpxb_engine_all_gather(void* engine, const void* in, void* out, uint64_t bytes_per_rank, void* stream);
 // reduce_scatter: `in` holds world x bytes_per_rank; out receives this rank's reduced part.
 int tcpxb_engine_reduce_scatter(void* engine, const void* in, void* out, uint64_t bytes_per_rank, int dtype, void* stream);
+// With one GPU per node the kernels take fragments of any length and phase, so the sizes above need not be multiples
+// of 16 bytes: after tcpxb_engine_set_ragged(engine, 1), whole elements are enough (all_reduce: between two nodes
+// only, a ring of more cuts pieces).  No effect with several GPUs per node or in plain_mode.
+int tcpxb_engine_set_ragged(void* engine, int on);
 // Point-to-point over rail 0..n to the next / from the previous node (same local index).
 int tcpxb_engine_send_next(void* engine, const void* buf, uint64_t bytes, void* stream);
 int tcpxb_engine_recv_prev(void* engine, void* buf, uint64_t bytes, void* stream);

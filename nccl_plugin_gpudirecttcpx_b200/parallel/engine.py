@@ -57,6 +57,7 @@ def bind_engine_api(lib):
     lib.tcpxb_engine_all_reduce.argtypes = [vp, vp, vp, u64, ci, vp]
     lib.tcpxb_engine_all_gather.argtypes = [vp, vp, vp, u64, vp]
     lib.tcpxb_engine_reduce_scatter.argtypes = [vp, vp, vp, u64, ci, vp]
+    lib.tcpxb_engine_set_ragged.argtypes = [vp, ci]
     lib.tcpxb_engine_send_next.argtypes = [vp, vp, u64, vp]
     lib.tcpxb_engine_recv_prev.argtypes = [vp, vp, u64, vp]
     for name in ("tcpxb_engine_all_reduce_async", "tcpxb_engine_reduce_scatter_async"):
@@ -153,6 +154,9 @@ class HierarchicalEngine:
         self._h = self._api.tcpxb_engine_create(ctypes.byref(cfg))
         if not self._h:
             raise RuntimeError("engine create failed: " + self._api.tcpxb_engine_last_error().decode())
+        # one GPU per node: the native calls take any whole number of elements, no padded copies are needed
+        self._ragged = self.G == 1 and not plain_mode
+        self._check(self._api.tcpxb_engine_set_ragged(self._h, int(self._ragged)))
         self.rails = self._api.tcpxb_engine_rails(self._h)
         self._connect()
         self.work = self.out = None
@@ -226,9 +230,20 @@ class HierarchicalEngine:
         more than two nodes, every piece of it) is a whole number of 16-byte vectors."""
         return self.G * (self.nodes if self.nodes > 2 else 1) * 16
 
+    def _takes_ragged(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> bool:
+        """True when the native call can read `x`, of any size, and write `out` where they are.  Layouts that the
+        padded copies put right (strides, another shape, type or device, a partial overlap) keep going through them."""
+        if not (self._ragged and x.numel() and x.is_contiguous() and x.device == self.device):
+            return False
+        if out is None or out.data_ptr() == x.data_ptr() and out.shape == x.shape and out.dtype == x.dtype and out.is_contiguous():
+            return True
+        nbytes = x.numel() * x.element_size()
+        apart = out.data_ptr() + nbytes <= x.data_ptr() or x.data_ptr() + nbytes <= out.data_ptr()
+        return apart and out.shape == x.shape and out.dtype == x.dtype and out.device == x.device and out.is_contiguous()
+
     def all_reduce(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """Sum over all ranks, any number of elements (sizes that are not a multiple of the
-        native granularity are zero-padded on the way in and trimmed on the way out).
+        """Sum over all ranks, any number of elements (where the native call needs a multiple of its
+        granularity, sizes are zero-padded on the way in and trimmed on the way out).
         G == 1: any contiguous tensors.  G > 1: `x` is staged into the symmetric work buffer
         and the result is a view of the symmetric output."""
         nbytes = x.numel() * x.element_size()
@@ -236,7 +251,7 @@ class HierarchicalEngine:
         unit = self._all_reduce_unit()
         padded = (nbytes + unit - 1) // unit * unit
         if self.G == 1:
-            if padded != nbytes:
+            if padded != nbytes and not (self.nodes == 2 and self._takes_ragged(x, out)):
                 xin = torch.zeros(padded // x.element_size(), dtype=x.dtype, device=x.device)
                 xin[:x.numel()].copy_(x.reshape(-1))
                 res = torch.empty_like(xin)
@@ -365,11 +380,11 @@ class HierarchicalEngine:
         return self.work.view(torch.uint8)[:numel * dtype.itemsize].view(dtype)
 
     def all_gather(self, x: torch.Tensor) -> torch.Tensor:
-        """Concatenation of every rank's `x` in rank order.  Blocks whose byte size is not a
-        multiple of 16 travel padded and are compacted on return."""
+        """Concatenation of every rank's `x` in rank order.  With several GPUs per node, blocks whose
+        byte size is not a multiple of 16 travel padded and are compacted on return."""
         nbytes = x.numel() * x.element_size()
         blocks = self.nodes * self.G
-        if nbytes % 16 != 0:
+        if nbytes % 16 != 0 and not self._takes_ragged(x):
             padded = (nbytes + 15) // 16 * 16
             xin = torch.zeros(padded, dtype=torch.uint8, device=x.device)
             xin[:nbytes].copy_(x.reshape(-1).view(torch.uint8))
@@ -386,14 +401,14 @@ class HierarchicalEngine:
 
     def reduce_scatter(self, x: torch.Tensor) -> torch.Tensor:
         """Sum over all ranks of `x`, of which this rank keeps its 1/world part (`x.numel()`
-        must divide by the number of ranks).  Parts whose byte size is not a multiple of 16
-        travel padded."""
+        must divide by the number of ranks).  With several GPUs per node, parts whose byte size is
+        not a multiple of 16 travel padded."""
         blocks = self.nodes * self.G if self.world > 1 else 1
         if x.numel() % blocks != 0:
             raise ValueError(f"reduce_scatter input of {x.numel()} elements does not divide into {blocks} parts")
         per = x.numel() // blocks
         nbytes = per * x.element_size()
-        if nbytes % 16 != 0:
+        if nbytes % 16 != 0 and not self._takes_ragged(x):
             per_padded = (nbytes + 15) // 16 * 16 // x.element_size()
             xin = torch.zeros(blocks, per_padded, dtype=x.dtype, device=x.device)
             xin[:, :per].copy_(x.reshape(blocks, per))
