@@ -231,9 +231,10 @@ class HierarchicalEngine:
         return self.G * (self.nodes if self.nodes > 2 else 1) * 16
 
     def _takes_ragged(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> bool:
-        """True when the native call can read `x`, of any size, and write `out` where they are.  Layouts that the
-        padded copies put right (strides, another shape, type or device, a partial overlap) keep going through them."""
-        if not (self._ragged and x.numel() and x.is_contiguous() and x.device == self.device):
+        """True when the native call can read `x`, of any size, and write `out` where they are.  Other layouts (strides,
+        another shape, type or device, a partial overlap) go through copies.  That is this rank's affair alone:
+        the bytes on the wire depend on the size only, since the other ranks' tensors may be laid out otherwise."""
+        if not (self._ragged and x.numel() and x.is_contiguous()):
             return False
         if out is None or out.data_ptr() == x.data_ptr() and out.shape == x.shape and out.dtype == x.dtype and out.is_contiguous():
             return True
@@ -251,11 +252,12 @@ class HierarchicalEngine:
         unit = self._all_reduce_unit()
         padded = (nbytes + unit - 1) // unit * unit
         if self.G == 1:
-            if padded != nbytes and not (self.nodes == 2 and self._takes_ragged(x, out)):
-                xin = torch.zeros(padded // x.element_size(), dtype=x.dtype, device=x.device)
+            wire = nbytes if self._ragged and self.nodes == 2 else padded
+            if padded != nbytes and not (wire == nbytes and self._takes_ragged(x, out)):
+                xin = torch.zeros(wire // x.element_size(), dtype=x.dtype, device=x.device)
                 xin[:x.numel()].copy_(x.reshape(-1))
                 res = torch.empty_like(xin)
-                self._check(self._api.tcpxb_engine_all_reduce(self._h, xin.data_ptr(), res.data_ptr(), padded, code, self._stream()))
+                self._check(self._api.tcpxb_engine_all_reduce(self._h, xin.data_ptr(), res.data_ptr(), wire, code, self._stream()))
                 res = res[:x.numel()].view(x.shape)
                 if out is not None:
                     out.copy_(res)
@@ -385,7 +387,7 @@ class HierarchicalEngine:
         nbytes = x.numel() * x.element_size()
         blocks = self.nodes * self.G
         if nbytes % 16 != 0 and not self._takes_ragged(x):
-            padded = (nbytes + 15) // 16 * 16
+            padded = nbytes if self._ragged else (nbytes + 15) // 16 * 16
             xin = torch.zeros(padded, dtype=torch.uint8, device=x.device)
             xin[:nbytes].copy_(x.reshape(-1).view(torch.uint8))
             g = self.all_gather(xin)
@@ -409,7 +411,7 @@ class HierarchicalEngine:
         per = x.numel() // blocks
         nbytes = per * x.element_size()
         if nbytes % 16 != 0 and not self._takes_ragged(x):
-            per_padded = (nbytes + 15) // 16 * 16 // x.element_size()
+            per_padded = per if self._ragged else (nbytes + 15) // 16 * 16 // x.element_size()
             xin = torch.zeros(blocks, per_padded, dtype=x.dtype, device=x.device)
             xin[:, :per].copy_(x.reshape(blocks, per))
             return self.reduce_scatter(xin.view(-1))[:per].clone()
