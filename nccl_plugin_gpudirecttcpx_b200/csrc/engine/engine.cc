@@ -302,7 +302,7 @@ int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_of
   uint32_t* done = e->kernel_marks.take(done_mark);
   const bool nvls = fan && e->cfg.use_nvls && e->mc_out != nullptr;
   ENG_K(tcpxb_unpack_request(sl.pool_dev, sl.pool_bytes, acc, dst, nvls ? e->mc_out + rs.out_offset + region_off : nullptr, len, peers,
-                             npeers, descs, count, rs.dtype, !fan && acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM, e->status_dev,
+                             npeers, descs, reinterpret_cast<const tcpxbLoadMeta*>(sl.host), count, rs.dtype, !fan && acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM, e->status_dev,
                              &opts, done, *done_mark, stream));
   return 0;
 }
@@ -323,6 +323,7 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
     // sends may read only what the stream has produced so far
     if (ss.bytes <= kStageKernelBytes && (reinterpret_cast<uintptr_t>(ss.src) & 15) == 0) {
       for (int r = 0; r < R; ++r) netSetSendStream(e->rails[r].send, stream);
+      e->stats.kernel_launches += n_send;  // one staging kernel per request
     } else {
       ENG_NET(gpu::eventRecord(e->dep_event, stream));
       for (int r = 0; r < R; ++r) netSetSendDependency(e->rails[r].send, e->dep_event);

@@ -133,12 +133,14 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
 // reduce (impl as for K2); the fan-out to `peers` when npeers > 0, through mc_dst when that is not
 // NULL.  The launch ends with *done_flag = done_value (release, system scope; mapped host memory),
 // errors or not, once every store of the launch is visible and every byte of the pool has been read.
-// opts->ticket is required.  An empty list launches nothing and writes nothing.
+// opts->ticket is required.  `descs_host`: the same records as the calling thread reads them, or NULL;
+// a short list then travels with the launch.  An empty list launches nothing and writes nothing.
 int tcpxb_unpack_request(const void* pool, uint64_t pool_bytes, const void* acc, void* dst,
                          void* mc_dst, uint64_t dst_bytes, void* const* peers, int npeers,
-                         const tcpxbLoadMeta* descs, uint32_t count, int dtype, int impl,
-                         uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag,
-                         uint32_t done_value, void* stream);
+                         const tcpxbLoadMeta* descs, const tcpxbLoadMeta* descs_host,
+                         uint32_t count, int dtype, int impl, uint32_t* status,
+                         const tcpxbUnpackOpts* opts, uint32_t* done_flag, uint32_t done_value,
+                         void* stream);
 
 // Loads every kernel of this library on the current device and applies their
 // launch attributes.  CUDA loads kernels lazily, and a first launch may have to

@@ -226,8 +226,8 @@ int tcpxb_unpack_reduce_fanout_nvls(const void* pool, uint64_t pool_bytes, const
 }
 
 int tcpxb_unpack_request(const void* pool, uint64_t pool_bytes, const void* acc, void* dst, void* mc_dst, uint64_t dst_bytes,
-                         void* const* peers, int npeers, const tcpxbLoadMeta* descs, uint32_t count, int dtype, int impl,
-                         uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag, uint32_t done_value, void* stream) {
+                         void* const* peers, int npeers, const tcpxbLoadMeta* descs, const tcpxbLoadMeta*, uint32_t count, int dtype,
+                         int impl, uint32_t* status, const tcpxbUnpackOpts* opts, uint32_t* done_flag, uint32_t done_value, void* stream) {
   if (done_flag == nullptr || opts == nullptr || opts->ticket == nullptr) return fail(TCPXB_K_INVALID, "a completion word and its ticket are needed");
   int rc;
   if (mc_dst != nullptr && acc != nullptr)
