@@ -21,8 +21,10 @@
 // pairs for the reduce), so an SM keeps 192 KB of loads in the air, which is what
 // HBM3e needs to stay busy with 4 KB transfers.  Twelve warps of depth 4 / 2
 // measured 2 - 3 % faster on the fused reduce than eight warps of depth 6 / 3.
-// Fragments whose addresses are not 16-byte aligned, or that are longer than a
-// slot, take a warp-cooperative ld/st path; ragged tails (< 16 B) likewise.
+// Fragments off the 16-byte phase and ragged ends come into the slot as the aligned
+// vectors that hold them and are stored by the warp; fragments longer than a slot take
+// a warp-cooperative ld/st path.  Long lists and a polling host's short ones go through
+// registers instead (unpack_wide_kernel, unpack_few_kernel).
 //
 // Every wait is bounded: on expiry the kernel records TCPXB_ST_TIMEOUT in the
 // status block, stops issuing, waits only for the loads already in flight and
