@@ -148,6 +148,8 @@ class HierarchicalEngine:
         self.world = self._dist.get_world_size() if self._dist else 1
         self.G = gpus_per_node
         self.device = device or torch.device("cuda", torch.cuda.current_device())
+        self._home = torch.device("cuda", self.device.index or 0) if self.device.type == "cuda" else self.device
+        self._home_index = -1 if self._home.index is None else self._home.index  # as Tensor.get_device() says it
         self.nodes = max(2, self.world // self.G) if self.world > 1 else 2
         cfg = _Config(self.rank, self.world, self.G, self.device.index or 0, request_bytes, max_inflight, unpack_ctas,
                       reduce_impl, int(use_nvls), int(plain_mode), idle_spin_us, idle_sleep_us, int(wake_on_events))
@@ -230,31 +232,37 @@ class HierarchicalEngine:
         more than two nodes, every piece of it) is a whole number of 16-byte vectors."""
         return self.G * (self.nodes if self.nodes > 2 else 1) * 16
 
-    def _takes_ragged(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> bool:
-        """True when the native call can read `x`, of any size, and write `out` where they are.  Other layouts (strides,
-        another shape, type or device, a partial overlap) go through copies.  That is this rank's affair alone:
-        the bytes on the wire depend on the size only, since the other ranks' tensors may be laid out otherwise."""
-        if not (self._ragged and x.numel() and x.is_contiguous()):
+    def _direct(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> bool:
+        """True when the native call can read `x` and write `out` where they are: contiguous, in memory the engine's GPU
+        addresses, `out` of the same type, large enough, and `x` itself or apart from it.  Other layouts go through
+        copies, at every size.  That is this rank's affair alone: the bytes on the wire depend on the size only, since
+        the other ranks' tensors may be laid out otherwise."""
+        home = self._home_index
+        if not (x.is_contiguous() and (x.get_device() == home or (out is not None and x.is_pinned()))):
             return False
-        if out is None or out.data_ptr() == x.data_ptr() and out.shape == x.shape and out.dtype == x.dtype and out.is_contiguous():
+        if out is None or out is x:
             return True
-        nbytes = x.numel() * x.element_size()
-        apart = out.data_ptr() + nbytes <= x.data_ptr() or x.data_ptr() + nbytes <= out.data_ptr()
-        return apart and out.shape == x.shape and out.dtype == x.dtype and out.device == x.device and out.is_contiguous()
+        if not (out.is_contiguous() and out.dtype is x.dtype and (out.get_device() == home or out.is_pinned())):
+            return False
+        nbytes = x.nbytes
+        apart = out.data_ptr() - x.data_ptr()
+        return out.nbytes >= nbytes and (apart == 0 or abs(apart) >= nbytes)
 
     def all_reduce(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Sum over all ranks, any number of elements (where the native call needs a multiple of its
-        granularity, sizes are zero-padded on the way in and trimmed on the way out).
-        G == 1: any contiguous tensors.  G > 1: `x` is staged into the symmetric work buffer
-        and the result is a view of the symmetric output."""
+        granularity, sizes are zero-padded on the way in and trimmed on the way out).  Contiguous tensors on the
+        engine's device are read and written where they are, others through copies.  G > 1: `x` is staged into the
+        symmetric work buffer and, without `out`, the result is a view of the symmetric output."""
         nbytes = x.numel() * x.element_size()
         code = DTYPE_CODE[x.dtype]
         unit = self._all_reduce_unit()
         padded = (nbytes + unit - 1) // unit * unit
+        # an `out` of another shape is written element by element in memory order if whole sizes allow it
+        direct = self._direct(x, out) and (padded == nbytes or out is None or out.shape == x.shape)
         if self.G == 1:
             wire = nbytes if self._ragged and self.nodes == 2 else padded
-            if padded != nbytes and not (wire == nbytes and self._takes_ragged(x, out)):
-                xin = torch.zeros(wire // x.element_size(), dtype=x.dtype, device=x.device)
+            if nbytes and not (direct and wire == nbytes):
+                xin = torch.zeros(wire // x.element_size(), dtype=x.dtype, device=self._home)
                 xin[:x.numel()].copy_(x.reshape(-1))
                 res = torch.empty_like(xin)
                 self._check(self._api.tcpxb_engine_all_reduce(self._h, xin.data_ptr(), res.data_ptr(), wire, code, self._stream()))
@@ -262,21 +270,21 @@ class HierarchicalEngine:
                 if out is not None:
                     out.copy_(res)
                     return out
-                return res
+                return res.to(x.device)
             if out is None:
                 out = torch.empty_like(x)
             self._check(self._api.tcpxb_engine_all_reduce(self._h, x.data_ptr(), out.data_ptr(), nbytes, code, self._stream()))
             return out
         if padded > self.buffer_bytes:
             raise ValueError(f"all_reduce of {nbytes} bytes does not fit the {self.buffer_bytes}-byte symmetric buffers")
-        if padded == nbytes and x.is_contiguous() and (out is None or out.is_contiguous()):
+        if padded == nbytes and direct:
             # the native call stages tensors that live outside the symmetric buffers itself
             dst = out.data_ptr() if out is not None else self.out.data_ptr()
             self._check(self._api.tcpxb_engine_all_reduce(self._h, x.data_ptr(), dst, nbytes, code, self._stream()))
             return out if out is not None else self.out.view(torch.uint8)[:nbytes].view(x.dtype).view(x.shape)
         wb = self.work.view(torch.uint8)
         w = wb[:nbytes].view(x.dtype)
-        if x.data_ptr() != w.data_ptr():
+        if x.data_ptr() != w.data_ptr() or not x.is_contiguous():
             w.copy_(x.reshape(-1))
         if padded != nbytes:
             wb[nbytes:padded].zero_()
@@ -386,12 +394,12 @@ class HierarchicalEngine:
         byte size is not a multiple of 16 travel padded and are compacted on return."""
         nbytes = x.numel() * x.element_size()
         blocks = self.nodes * self.G
-        if nbytes % 16 != 0 and not self._takes_ragged(x):
+        if nbytes and not (self._direct(x) and (nbytes % 16 == 0 or self._ragged)):
             padded = nbytes if self._ragged else (nbytes + 15) // 16 * 16
-            xin = torch.zeros(padded, dtype=torch.uint8, device=x.device)
+            xin = torch.zeros(padded, dtype=torch.uint8, device=self._home)
             xin[:nbytes].copy_(x.reshape(-1).view(torch.uint8))
             g = self.all_gather(xin)
-            return g.view(blocks, padded)[:, :nbytes].contiguous().view(-1).view(x.dtype)
+            return g.view(blocks, padded)[:, :nbytes].contiguous().view(-1).view(x.dtype).to(x.device)
         if self.G == 1:
             out = torch.empty(blocks * x.numel(), dtype=x.dtype, device=x.device)
             self._check(self._api.tcpxb_engine_all_gather(self._h, x.data_ptr(), out.data_ptr(), nbytes, self._stream()))
@@ -410,18 +418,19 @@ class HierarchicalEngine:
             raise ValueError(f"reduce_scatter input of {x.numel()} elements does not divide into {blocks} parts")
         per = x.numel() // blocks
         nbytes = per * x.element_size()
-        if nbytes % 16 != 0 and not self._takes_ragged(x):
+        whole = nbytes % 16 == 0
+        if nbytes and not (whole if self.G > 1 else self._direct(x) and (whole or self._ragged)):
             per_padded = per if self._ragged else (nbytes + 15) // 16 * 16 // x.element_size()
-            xin = torch.zeros(blocks, per_padded, dtype=x.dtype, device=x.device)
+            xin = torch.zeros(blocks, per_padded, dtype=x.dtype, device=self._home)
             xin[:, :per].copy_(x.reshape(blocks, per))
-            return self.reduce_scatter(xin.view(-1))[:per].clone()
+            return self.reduce_scatter(xin.view(-1))[:per].clone().to(x.device)
         out = torch.empty(per, dtype=x.dtype, device=x.device)
         src = x
         if self.G > 1:
             if x.numel() * x.element_size() > self.buffer_bytes:
                 raise ValueError(f"reduce_scatter input of {x.numel() * x.element_size()} bytes does not fit the symmetric buffers")
             w = self.work.view(torch.uint8)[:x.numel() * x.element_size()].view(x.dtype)
-            if x.data_ptr() != w.data_ptr():
+            if x.data_ptr() != w.data_ptr() or not x.is_contiguous():
                 w.copy_(x.reshape(-1))
             src = self.work
         self._check(self._api.tcpxb_engine_reduce_scatter(self._h, src.data_ptr(), out.data_ptr(), nbytes, DTYPE_CODE[x.dtype], self._stream()))

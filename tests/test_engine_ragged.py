@@ -77,3 +77,25 @@ def test_native_sizes_stay_checked(engine):
         assert engine._api.tcpxb_engine_reduce_scatter(engine._h, x.data_ptr(), y.data_ptr(), 12, 2, None) != 0
     finally:
         engine._api.tcpxb_engine_set_ragged(engine._h, 1)
+
+
+def test_layouts_at_whole_sizes(engine):
+    """The same at sizes that need no padding, and an output of the wrong size is refused before anything is written."""
+    base = torch.randint(-64, 64, (2 * 1008,), device="cuda").float()
+    strided = base.view(2, 1008).t()
+    assert torch.equal(engine.all_reduce(strided), strided * 2)
+    assert torch.equal(engine.all_gather(strided), torch.cat([strided, strided]).reshape(-1))
+    assert torch.equal(engine.reduce_scatter(strided), (strided * 2).reshape(-1))
+    want = base[:1008] * 2
+    wide = torch.empty(1008, dtype=torch.float64, device="cuda")
+    assert engine.all_reduce(base[:1008], wide) is wide and torch.equal(wide, want.double())
+    on_host = torch.empty(1008)
+    assert engine.all_reduce(base[:1008], on_host) is on_host and torch.equal(on_host, want.cpu())
+    assert torch.equal(engine.all_reduce(base[:1008].cpu()), want.cpu())
+    room = torch.full((1008,), 7.0, device="cuda")
+    with pytest.raises(RuntimeError):
+        engine.all_reduce(base[:1008], room[:512])
+    assert (room == 7).all()
+    shifted = base[16:1024]
+    assert engine.all_reduce(base[:1008], shifted) is shifted and torch.equal(shifted, want)
+    assert engine.device_status()[0] == 0
