@@ -315,6 +315,8 @@ class HierarchicalEngine:
         unit = self._all_reduce_unit()
         if nbytes % unit != 0 or not x.is_contiguous() or (out is not None and not out.is_contiguous()):
             raise ValueError(f"all_reduce_async needs contiguous tensors whose size is a multiple of {unit} bytes")
+        if out is not None and out.nbytes < nbytes:
+            raise ValueError(f"out must hold {nbytes} bytes")
         if self.G == 1:
             res = out if out is not None else torch.empty_like(x)
             src, dst = x.data_ptr(), res.data_ptr()

@@ -51,6 +51,11 @@ for cols in (16, 1024):
         raise SystemExit("an output that is too small was taken")
     except RuntimeError:
         assert (room == 7).all(), "written past the end of the output"
+    try:
+        eng.all_reduce_async(a, room[:rows * cols // 2]).wait()
+        raise SystemExit("an output that is too small was taken")
+    except ValueError:
+        assert (room == 7).all(), "written past the end of the output"
     assert torch.equal(eng.all_gather(mine), torch.cat([t.reshape(-1) for t in ins]))
     parts = ranks if world > 1 else 1
     assert torch.equal(eng.reduce_scatter(mine), total.reshape(parts, -1)[rank])
