@@ -83,8 +83,10 @@ typedef struct tcpxbUnpackOpts {
   // Programmatic dependent launch: the launch may be scheduled while the previous kernel
   // of the stream is still running; its CTAs become resident as SMs free up, set up
   // their barriers, and wait for that kernel to complete (and its writes to be visible)
-  // before they touch any memory.  Every launch is made that way; the field is accepted
-  // for callers that ask for it.
+  // before they touch any memory.  Every launch is made that way, and one over the whole GPU
+  // lets its successor in at once.  A launch confined by max_ctas does that only if this is
+  // non-zero, else when its work is done: a waiting successor holds SMs beyond the cap.  A
+  // streamed launch (ready_count) lets nothing in before its last record is through.
   int early_launch;
 } tcpxbUnpackOpts;
 

@@ -79,6 +79,7 @@ struct UnpackParams {
   uint32_t* status;
   const uint32_t* ready;
   uint64_t wait_ns;
+  uint32_t let_in;  // the next launch may come in once this one is past its own wait; 0: once its work is done
 };
 
 struct SlotInfo {
@@ -458,18 +459,16 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kDataBytes) + warp * C::kDepth;
   SlotInfo* infos = reinterpret_cast<SlotInfo*>(smem + C::kDataBytes + kWarps * C::kDepth * 8) + warp * C::kDepth;
 
-  // Programmatic dependent launch, both roles.  As the earlier kernel: let a dependent
-  // launch be scheduled from now on (its CTAs still need this one's shared memory to
-  // be released before they fit).  As the later kernel: everything up to the wait
-  // below touches only this CTA's shared memory; the wait returns when the previous
-  // kernel of the stream has completed and its writes are visible.
-  pdl_launch_dependents();
+  // Programmatic dependent launch.  As the later kernel: everything up to the wait below
+  // touches only this CTA's shared memory; the wait returns when the previous kernel of the
+  // stream has completed and its writes are visible.  As the earlier one: see launchDependent.
   __shared__ uint32_t cta_err;  // any warp of this CTA recorded an error
   if (threadIdx.x == 0) cta_err = 0;
   if (lane < (int)D) mbar_init(smem_u32(&bars[lane]), 1);
   fence_mbar_init();
   __syncthreads();
   pdl_wait();
+  if (p.let_in) pdl_launch_dependents();
   auto record = [&](uint32_t code, uint32_t index) {  // one lane calls this
     report(p.status, code, index);
     atomicOr(&cta_err, 1u);
@@ -665,6 +664,10 @@ unpack_kernel(const __grid_constant__ UnpackParams p) {
     }
   }
   if (lane == 0) bulk_wait_all();
+  if (!p.let_in) {
+    __syncthreads();  // the first thread to say so speaks for the whole CTA
+    pdl_launch_dependents();
+  }
 
   if ((p.flag_value != 0 || p.done_flag != nullptr) && p.ticket != nullptr) {
     // Publish completion once every CTA's stores are done: to the peers (unless there were errors), and to
@@ -818,10 +821,10 @@ template <int RED>
 __global__ void __launch_bounds__(kWideThreads, RED == TCPXB_U8 ? 4 : 3)
 unpack_wide_kernel(const __grid_constant__ UnpackParams p) {
   const uint32_t idx = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // neighbours in the list go to different SMs
-  pdl_launch_dependents();
   const uint64_t pool_policy = policy_evict_first();
   if (idx >= p.count) return;
   pdl_wait();
+  pdl_launch_dependents();
   wide_record<RED>(p, ld_v4(&p.descs[idx]), idx, pool_policy, threadIdx.x & 31);
 }
 
@@ -837,7 +840,6 @@ struct FewParams {
 template <int RED>
 __global__ void __launch_bounds__(kWideThreads, 1) unpack_few_kernel(const __grid_constant__ FewParams q) {
   const uint32_t warp = threadIdx.x >> 5;
-  pdl_launch_dependents();
   const uint64_t pool_policy = policy_evict_first();
   pdl_wait();
   if (warp < q.p.count) wide_record<RED>(q.p, q.recs[warp], warp, pool_policy, threadIdx.x & 31);
@@ -851,7 +853,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) unpack_few_kernel(const __gri
 // Bounded wait for peer completion flags; one warp, lane i watches flags[i].
 __global__ void wait_flags_kernel(const uint32_t* flags, int n, uint32_t value, uint64_t wait_ns,
                                   uint32_t* status) {
-  // A kernel behind this one is let in only at its end: it would hold SMs while this one waits for a peer.
+  // Lets nothing in: a kernel behind this one would hold SMs while this one waits for a peer.
   const int i = threadIdx.x;
   pdl_wait();
   if (i >= n) return;
@@ -874,8 +876,8 @@ struct SignalParams {
 };
 __global__ void signal_flags_kernel(const __grid_constant__ SignalParams p) {
   const int i = threadIdx.x;
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (i < p.n && p.flags[i] != nullptr) {
     __threadfence_system();
     st_release_sys(p.flags[i], p.value);
@@ -890,7 +892,6 @@ constexpr int kStageThreads = 1024;
 __global__ void __launch_bounds__(kStageThreads)
 stage_out_kernel(const uint8_t* src, uint8_t* dst, uint64_t bytes, uint32_t* flag, uint32_t value) {
   const uint64_t vecs = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? bytes >> 4 : 0;
-  pdl_launch_dependents();
   pdl_wait();
 #pragma unroll 4
   for (uint64_t i = threadIdx.x; i < vecs; i += blockDim.x) *reinterpret_cast<uint4*>(dst + (i << 4)) = ld_v4(src + (i << 4));
@@ -957,10 +958,10 @@ constexpr int kFewSources = 4;
 template <int RED, int N, bool WIDE>
 __global__ void __launch_bounds__(kPeerThreads) peer_reduce_kernel(const __grid_constant__ PeerReduceParams p) {
   const uint64_t i = ((uint64_t)blockIdx.x * kPeerThreads + threadIdx.x) * (WIDE ? 2 : 1);
-  pdl_launch_dependents();
   if (i >= p.vecs) return;
   const uint64_t off = p.shard_off + (i << 4);
   pdl_wait();
+  pdl_launch_dependents();
   if (WIDE && i + 1 < p.vecs) {
     uint4 lo[N], hi[N];
 #pragma unroll
@@ -991,8 +992,8 @@ struct CsumScratch {
 };
 __global__ void __launch_bounds__(kCsumThreads)
 checksum_kernel(const uint8_t* buf, uint64_t bytes, uint64_t* out, CsumScratch* scratch) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const uint64_t words = bytes >> 2;
   const uint32_t* w = reinterpret_cast<const uint32_t*>(buf);
   uint64_t sum = 0;
@@ -1113,9 +1114,16 @@ int deviceInfo(int* dev_out) {
   return TCPXB_K_OK;
 }
 
-// Every launch may be scheduled while its predecessor in the stream still runs (programmatic
-// dependent launch): the kernels wait for that predecessor on the device before they touch any
-// memory, so results do not change and back-to-back launches lose about 0.6 us each.
+// Every launch may be scheduled while its predecessor in the stream still runs (programmatic dependent launch): the
+// kernels wait for that predecessor on the device before they touch any memory, so results do not change and
+// back-to-back launches save about 0.6 us each.  When a predecessor lets it in is that kernel's affair, since what
+// waiting CTAs hold is not free for other streams:
+//  - only after its own wait: at most one launch of a stream waits at a time, and a successor that reads something
+//    before it waits still finds all that was written up to the kernel before this one;
+//  - a kernel that waits for the host or another GPU (streamed records, flags), or that keeps to a part of the GPU, lets
+//    its successor in when its work is done or not at all: that successor could take the SMs which the producer, or the
+//    work beside a confined launch, needs.  At the end is early enough: 1 MiB requests on 16 CTAs, back to back, take
+//    25.0 us with it as with a successor let in at once, 26.6 us if launched without.
 template <typename Kernel, typename... Args>
 int launchDependent(Kernel kernel, unsigned ctas, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -1142,7 +1150,7 @@ int launch(const UnpackParams& p, int max_ctas, cudaStream_t stream) {
   if (rc) return rc;
   if (p.count == 0) return TCPXB_K_OK;
   const int sms = g_dev[dev].sms;
-  const bool whole_gpu = max_ctas <= 0 || max_ctas >= sms;
+  const bool whole_gpu = max_ctas <= 0 || max_ctas >= sms, asked = p.let_in != 0;
   if constexpr (FAN == FAN_NONE && !L2RED) {
     // Up to one record per ring warp the ring kernel is ahead (4 MiB in pages: 2.4 against 3.2 us, its bulk
     // copies need one instruction per page); beyond that its second, part-filled round costs more than it saves.
@@ -1154,7 +1162,9 @@ int launch(const UnpackParams& p, int max_ctas, cudaStream_t stream) {
   // them on one SM share its bulk-copy engine (256 records: 3.1 us on 22 SMs, 2.3 us on 148).
   const int cap = whole_gpu ? sms : max_ctas;
   const int ctas = p.count < (uint32_t)cap ? (int)p.count : cap;
-  return launchDependent(unpack_kernel<RED, L2RED, FAN>, (unsigned)ctas, kThreads, C::kSmemBytes, stream, p);
+  UnpackParams q = p;
+  q.let_in = p.ready == nullptr && (whole_gpu || asked) ? 1 : 0;
+  return launchDependent(unpack_kernel<RED, L2RED, FAN>, (unsigned)ctas, kThreads, C::kSmemBytes, stream, q);
 }
 
 // Device address of the allocation-free checksum's scratch on `dev` (the current
@@ -1231,6 +1241,7 @@ int fill(UnpackParams& p, const void* pool, uint64_t pool_bytes, const void* acc
   p.status = status;
   if (opts != nullptr) {
     p.ready = opts->ready_count;
+    p.let_in = opts->early_launch != 0;
     p.wait_ns = opts->wait_ns;
     p.flag_value = opts->flag_value;
     p.ticket = opts->ticket;

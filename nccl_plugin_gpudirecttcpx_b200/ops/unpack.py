@@ -151,7 +151,7 @@ def _opts(ready_count=None, wait_ns=0, peer_flags: Sequence[int] = (), flag_valu
     o.flag_value = int(flag_value)
     o.ticket = None if ticket is None else ticket.data_ptr()
     o.max_ctas = int(max_ctas)
-    o.early_launch = int(bool(early_launch))  # programmatic dependent launch: may start while the stream's previous kernel still runs
+    o.early_launch = int(bool(early_launch))  # whole-GPU launches let their successor start early in any case, one confined by max_ctas with this
     return o, ctypes.byref(o)
 
 
