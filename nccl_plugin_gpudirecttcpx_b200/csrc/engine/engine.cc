@@ -25,6 +25,7 @@
 #include <nvtx3/nvToolsExt.h>
 #endif
 
+#include "tcpxb/cpu_budget.h"
 #include "tcpxb/kernels.h"
 #include "tcpxb/transport.h"
 
@@ -54,16 +55,6 @@ int fail(const char* fmt, const char* a = "", long b = 0) {
   do {                                                                          \
     if ((expr) != 0) return -1;                                                 \
   } while (0)
-
-// Cores this process may use, shared with the other ranks of the box (the launcher's LOCAL_WORLD_SIZE).
-int coresPerRank() {
-  cpu_set_t set;
-  CPU_ZERO(&set);
-  if (sched_getaffinity(0, sizeof set, &set) != 0) return 1;
-  const char* v = getenv("LOCAL_WORLD_SIZE");
-  const int ranks = v != nullptr ? atoi(v) : 1;
-  return CPU_COUNT(&set) / std::max(1, ranks);
-}
 
 double nowSec() {
   struct timespec ts;
@@ -137,6 +128,7 @@ struct Engine {
   // idle policy of the driving thread
   Notifier notifier;
   int idle_spin_us = 20, idle_sleep_us = 30;
+  int local_ranks = 1;       // see tcpxb_engine_set_local_ranks
   bool spare_cores = false;  // a core for the driving thread beside the helper threads'
   bool wake_on_events = false;  // sleep in ppoll on the control sockets and an eventfd instead of napping
   // asynchronous calls: jobs run in order on a thread and a stream of the engine's own
@@ -163,9 +155,8 @@ constexpr double kSmallExchangeSpinUs = 250.0;
 // With cores to spare the driving thread looks for the next event this long before it naps: a nap of
 // 30 us ends 50 us and more later, once the timer and the scheduler are through.  Nap -> spin, all_reduce in us:
 // 16 cores, 1 MiB 162 -> 131, 4 MiB 423 -> 359, 16 MiB 950 -> 861, 256 MiB 11.9 -> 11.7 ms; 12 cores, the same up to
-// 16 MiB but 25 MiB 1348 -> 1454 and 64 MiB 3088 -> 3239; 4 cores, 4 MiB 580 -> 3746.  Hence the line at 16.
+// 16 MiB but 25 MiB 1348 -> 1454 and 64 MiB 3088 -> 3239; 4 cores, 4 MiB 580 -> 3746.  Hence the line at 16 (spareCores).
 constexpr double kSpareCoreSpinUs = 1000.0;
-constexpr int kSpareCores = 16;
 constexpr int64_t kLeastChunk = 128 << 10;
 constexpr double kLastKernelSpinUs = 200.0;
 // Up to here a whole exchange is staged by kernels on the caller's stream, where they queue before its unpack kernels.
@@ -609,7 +600,6 @@ void* tcpxb_engine_create(const tcpxbEngineConfig* cfg) {
   if (cfg->idle_spin_us > 0) e->idle_spin_us = cfg->idle_spin_us;
   if (cfg->idle_sleep_us != 0) e->idle_sleep_us = cfg->idle_sleep_us;
   e->wake_on_events = cfg->wake_on_events != 0;
-  e->spare_cores = cfg->idle_sleep_us == 0 && !e->wake_on_events && coresPerRank() >= kSpareCores;
   if (e->wake_on_events) e->notifier.event_fd = eventfd(0, EFD_NONBLOCK | EFD_CLOEXEC);
   prctl(PR_SET_TIMERSLACK, 1, 0, 0, 0);  // naps are tens of microseconds: no 50 us default slack on this thread
   int ndev = 0;
@@ -701,7 +691,18 @@ int tcpxb_engine_connect(void* engine, const void* next_handles) {
       netSetNotifier(rail.recv, &e->notifier);
     }
   }
+  int helpers = 0;
+  for (const Rail& rail : e->rails) helpers += rail.send->num_threads + rail.recv->num_threads;
+  e->spare_cores = e->cfg.idle_sleep_us == 0 && !e->wake_on_events &&
+                   spareCores(usableCores(), localRanks(e->G, e->local_ranks), helpers);
   e->connected = true;
+  return 0;
+}
+
+int tcpxb_engine_set_local_ranks(void* engine, int ranks) {
+  Engine* e = static_cast<Engine*>(engine);
+  if (e == nullptr || ranks < 1) return fail("no engine, or a number of ranks below one%s", "");
+  e->local_ranks = ranks;
   return 0;
 }
 

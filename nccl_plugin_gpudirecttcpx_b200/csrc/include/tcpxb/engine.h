@@ -80,6 +80,9 @@ int tcpxb_engine_listen(void* engine, void* handles_out);
 // Connects to the next node's handles and accepts the previous node's connection.
 // `next_handles` are the bytes the next neighbour's tcpxb_engine_listen produced.
 int tcpxb_engine_connect(void* engine, const void* next_handles);
+// Before tcpxb_engine_connect: how many ranks share this box's cores, where the caller knows of more than the launcher's
+// LOCAL_WORLD_SIZE and gpus_per_node say.  The driving thread spins at length only where each has cores to spare.
+int tcpxb_engine_set_local_ranks(void* engine, int ranks);
 // Intra-node peer mappings, all indexed by local rank (the own entry included):
 // work buffers (inputs are staged here), output buffers, flag blocks
 // (>= 64 uint32 each, zero-initialised) and optionally a multicast mapping of the

@@ -8,6 +8,7 @@
 // untested: ring cursor algebra, both flow mappers, control-record coalescing,
 // the stall detector on an injected clock, flag parsing and range fallback,
 // interface-list syntax, the page allocator and the scatter-list ring.
+#include <limits.h>
 #include <stdio.h>
 #include <sys/time.h>
 #include <stdlib.h>
@@ -15,6 +16,7 @@
 #include <linux/errqueue.h>
 #include <netinet/in.h>
 #include <sys/socket.h>
+#include <sys/stat.h>
 #include <sys/wait.h>
 #include <unistd.h>
 
@@ -26,6 +28,7 @@
 #include <thread>
 #include <vector>
 
+#include "tcpxb/cpu_budget.h"
 #include "tcpxb/ctrl_sock.h"
 #include "tcpxb/cu_driver.h"
 #include "tcpxb/dev_queue.h"
@@ -1118,6 +1121,46 @@ TEST(shared_device_allocation_and_dmabuf_export_on_standin_device) {
   cu::sharedRelease(&client);
   cu::sharedRelease(&owner);
   EXPECT(owner.dptr == nullptr && client.dptr == nullptr);
+}
+
+TEST(cpu_budget_sees_quotas_and_ranks) {
+  char dir[] = "/tmp/tcpxb_cgroup_XXXXXX";
+  EXPECT(mkdtemp(dir) != nullptr);
+  const std::string root = dir;
+  auto put = [&](const std::string& rel, const char* text) {
+    const std::string path = root + rel;
+    for (size_t i = root.size() + 1; (i = path.find('/', i)) != std::string::npos; ++i) mkdir(path.substr(0, i).c_str(), 0755);
+    FILE* f = fopen(path.c_str(), "w");
+    EXPECT(f != nullptr);
+    if (f != nullptr) { fputs(text, f); fclose(f); }
+  };
+  EXPECT(cgroupCpuLimit("0::/\n", root) == INT_MAX);  // no file: no quota
+  put("/job/cpu.max", "max 100000\n");
+  EXPECT(cgroupCpuLimit("0::/job\n", root) == INT_MAX);
+  put("/job/task/cpu.max", "650000 100000\n");
+  EXPECT(cgroupCpuLimit("0::/job/task\n", root) == 6);
+  put("/job/cpu.max", "400000 100000\n");  // the group above allows less
+  EXPECT(cgroupCpuLimit("0::/job/task\n", root) == 4);
+  EXPECT(cgroupCpuLimit("0::/job/other/not/there\n", root) == 4);
+  put("/job/task/cpu.max", "5000 100000\n");
+  EXPECT(cgroupCpuLimit("0::/job/task\n", root) == 1);
+  put("/cpu/box/cpu.cfs_quota_us", "-1\n");
+  put("/cpu/box/cpu.cfs_period_us", "100000\n");
+  EXPECT(cgroupCpuLimit("3:cpuset:/box\n1:cpu,cpuacct:/box\n0::/\n", root) == INT_MAX);
+  put("/cpu/box/cpu.cfs_quota_us", "300000\n");
+  EXPECT(cgroupCpuLimit("3:cpuset:/box\n1:cpu,cpuacct:/box\n0::/\n", root) == 3);
+  EXPECT(cgroupCpuLimit("3:cpuset:/box\n0::/\n", root) == INT_MAX);  // another controller's group says nothing about time
+  EXPECT(usableCores() >= 1);
+  // ranks: launchers that set nothing are covered by what the engine itself knows
+  unsetenv("LOCAL_WORLD_SIZE");
+  EXPECT(localRanks(1, 1) == 1 && localRanks(4, 1) == 4 && localRanks(1, 8) == 8);
+  setenv("LOCAL_WORLD_SIZE", "6", 1);
+  EXPECT(localRanks(4, 2) == 6 && localRanks(1, 8) == 8);
+  setenv("LOCAL_WORLD_SIZE", "0", 1);
+  EXPECT(localRanks(1, 1) == 1);
+  unsetenv("LOCAL_WORLD_SIZE");
+  EXPECT(spareCores(16, 1, 32) && spareCores(32, 2, 8) && spareCores(64, 1, 128));
+  EXPECT(!spareCores(15, 1, 8) && !spareCores(32, 8, 8) && !spareCores(16, 1, 33) && !spareCores(4, 1, 32));
 }
 
 TEST(chunk_size_follows_the_sockets) {

@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import socket
 from typing import Optional
 
 import torch
@@ -53,6 +54,7 @@ def bind_engine_api(lib):
     lib.tcpxb_engine_rails.argtypes = [vp]
     lib.tcpxb_engine_listen.argtypes = [vp, vp]
     lib.tcpxb_engine_connect.argtypes = [vp, vp]
+    lib.tcpxb_engine_set_local_ranks.argtypes = [vp, ci]
     lib.tcpxb_engine_set_peers.argtypes = [vp, vp, vp, vp, vp, u64]
     lib.tcpxb_engine_all_reduce.argtypes = [vp, vp, vp, u64, ci, vp]
     lib.tcpxb_engine_all_gather.argtypes = [vp, vp, vp, u64, vp]
@@ -102,6 +104,15 @@ def default_transport_env(nics: int = 4, nthreads: int = 4, nsocks_per_thread: i
         "NCCL_GPUDIRECTTCPX_CUDA_BUFFERS": "1",
     }.items():
         os.environ.setdefault(k, v)
+
+
+def _box_id() -> str:
+    """The same on every rank of a box, containers included."""
+    try:
+        with open("/proc/sys/kernel/random/boot_id") as f:
+            return f.read().strip()
+    except OSError:
+        return socket.gethostname()
 
 
 class AsyncWork:
@@ -187,9 +198,12 @@ class HierarchicalEngine:
             nxt = mine.raw
         else:
             allh = [None] * self.world
-            self._dist.all_gather_object(allh, mine.raw)
+            box = _box_id()
+            self._dist.all_gather_object(allh, (mine.raw, box))
             node, local = divmod(self.rank, self.G)
-            nxt = allh[((node + 1) % (self.world // self.G)) * self.G + local]
+            nxt = allh[((node + 1) % (self.world // self.G)) * self.G + local][0]
+            # not every launcher says how many ranks share a box
+            self._check(self._api.tcpxb_engine_set_local_ranks(self._h, sum(b == box for _, b in allh)))
         buf = ctypes.create_string_buffer(nxt, len(nxt))
         self._check(self._api.tcpxb_engine_connect(self._h, buf))
 

@@ -139,3 +139,22 @@ def test_bench_rails_and_threads_follow_the_cores():
     assert bench.rails_and_threads(32, 8) == (4, 1)     # 4 cores per rank: helpers sleep when idle, 4 rails still win
     assert bench.rails_and_threads(2, 8) == (1, 1)
     assert bench.rails_and_threads(32, 8, nics=2) == (2, 1) and bench.rails_and_threads(32, 8, nthreads=3) == (4, 3)
+
+
+def test_engine_learns_how_many_ranks_share_the_box():
+    """Launchers other than torchrun need not set LOCAL_WORLD_SIZE: the ranks count themselves while they connect."""
+    from types import SimpleNamespace
+    from nccl_plugin_gpudirecttcpx_b200.parallel.engine import HierarchicalEngine
+
+    def gather(out, mine):
+        for r in range(len(out)):
+            out[r] = mine if r < 3 else (mine[0], "another box")
+
+    told = []
+    eng = object.__new__(HierarchicalEngine)
+    eng._h, eng.rails, eng.rank, eng.world, eng.G = None, 1, 0, 8, 2
+    eng._dist = SimpleNamespace(all_gather_object=gather)
+    eng._api = SimpleNamespace(tcpxb_engine_listen=lambda h, b: 0, tcpxb_engine_connect=lambda h, b: 0,
+                               tcpxb_engine_set_local_ranks=lambda h, n: told.append(n) or 0)
+    eng._connect()
+    assert told == [3]
