@@ -456,10 +456,14 @@ int exchange(Engine* e, const SendSpec& ss, const RecvSpec& rs, void* stream) {
   for (int r = 0; r < R; ++r) any_left = any_left || !uq[r].empty();
   if (any_left) {
     // The last kernels end within tens of microseconds, and their counter says so sooner than a stream
-    // synchronise returns.  A kernel that failed never writes it: the stream has the reason.
+    // synchronise returns.  A kernel that failed never writes it: the stream has the reason.  Where the loop above
+    // would not spin, neither does this one.
     const uint32_t last = e->kernel_marks.issued();
-    const double t1 = nowSec();
-    while (!e->kernel_marks.reached(last) && (nowSec() - t1) * 1e6 < kLastKernelSpinUs) __builtin_ia32_pause();
+    const double limit = e->idle_sleep_us > 0 ? std::min(spin_us, kLastKernelSpinUs) : kLastKernelSpinUs, t1 = nowSec();
+    while (!e->kernel_marks.reached(last) && (nowSec() - t1) * 1e6 < limit) {
+      if (e->yield_when_idle) sched_yield();
+      else __builtin_ia32_pause();
+    }
     if (!e->kernel_marks.reached(last)) ENG_NET(gpu::streamSynchronize(stream));
   }
   for (int r = 0; r < R; ++r) {
