@@ -239,7 +239,7 @@ class HierarchicalEngine:
 
     # -------------------------------------------------------------- collectives
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return torch._C._cuda_getCurrentRawStream(self._home_index)  # without building a Stream object
 
     def _all_reduce_unit(self) -> int:
         """Byte granularity of the native all_reduce: every GPU's shard (and, on a ring of
