@@ -157,7 +157,6 @@ constexpr double kSmallExchangeSpinUs = 250.0;
 // 16 cores, 1 MiB 162 -> 131, 4 MiB 423 -> 359, 16 MiB 950 -> 861, 256 MiB 11.9 -> 11.7 ms; 12 cores, the same up to
 // 16 MiB but 25 MiB 1348 -> 1454 and 64 MiB 3088 -> 3239; 4 cores, 4 MiB 580 -> 3746.  Hence the line at 16 (spareCores).
 constexpr double kSpareCoreSpinUs = 1000.0;
-constexpr int64_t kLeastChunk = 128 << 10;
 constexpr double kLastKernelSpinUs = 200.0;
 // Up to here a whole exchange is staged by kernels on the caller's stream, where they queue before its unpack kernels.
 // Larger ones overlap staging with unpacking, which needs a stream of its own, and the copy engine takes no SM for it.
@@ -680,8 +679,9 @@ int tcpxb_engine_connect(void* engine, const void* next_handles) {
   for (Rail& rail : e->rails) {
     // staging no larger than what can be in flight: a small ring stays cache-resident
     const uint64_t want = (uint64_t)(e->inflight + 1) * (uint64_t)e->req_bytes;
-    // a request of 256 KiB on two sockets instead of one: all_reduce 87 -> 75 us, of 1 MiB 177 -> 162, of 4 MiB 453 -> 423
-    netSetLeastChunk(rail.send, kLeastChunk);
+    // with 128 KiB instead of 512, a request of 256 KiB goes over two sockets instead of one: all_reduce 87 -> 75 us, of
+    // 1 MiB 177 -> 162, of 4 MiB 453 -> 423
+    if (flags().engine_least_chunk > 0) netSetLeastChunk(rail.send, flags().engine_least_chunk);
     netSetTxStagingBytes(rail.send, std::min<uint64_t>(want, (uint64_t)flags().tx_staging_bytes));
     ENG_NET(netPrepareCuda(rail.send, e->cfg.gpu_dev));
     ENG_NET(netPrepareCuda(rail.recv, e->cfg.gpu_dev));

@@ -91,6 +91,7 @@ struct Flags {
   int64_t connect_pacing_us = 0;       // CONNECT_PACING_US per socket (the reference sleeps 100 ms)
   int64_t nic_speed_mbps = 0;          // NIC_SPEED_MBPS override for getProperties (0 = sysfs, else 10000)
   int64_t cuda_buffers = 0;            // CUDA_BUFFERS: accept CUDA pointers in host receive mode (see transport.h)
+  int64_t engine_least_chunk = 0;      // ENGINE_LEAST_CHUNK: quantum of the collective engine's own comms
   int64_t adaptive_chunk = 1;          // ADAPTIVE_CHUNK: about one chunk per socket and message (see chunkBytesFor)
   int64_t helper_nap_us = 0;           // HELPER_NAP_US: idle helper threads nap this long at a time (0 = off; the engine turns it on for its comms) ...
   int64_t helper_nap_rounds = 50;      // HELPER_NAP_ROUNDS: ... this many times before they sleep until woken

@@ -89,10 +89,14 @@ from .plugin_env import LOOPBACK_SNDBUF, loopback_sndbuf  # noqa: E402,F401
 
 def default_transport_env(nics: int = 4, nthreads: int = 4, nsocks_per_thread: int = 1,
                           chunk_bytes: int = 512 * 1024, pool_mb: int = 1024, sndbuf: int = -1) -> None:
-    """Environment defaults for the transport under the engine (only where unset).  `sndbuf`: SO_SNDBUF of
+    """Environment defaults for the transport under the engine (only where unset).  `chunk_bytes`: striping quantum; unless
+    the environment has one of its own, the engine's requests are cut down to 128 KiB where that occupies more sockets
+    (NCCL_GPUDIRECTTCPX_ENGINE_LEAST_CHUNK=0 keeps to the quantum).  `sndbuf`: SO_SNDBUF of
     the data sockets; -1 = `loopback_sndbuf` for this box's cores per rank (affinity mask / LOCAL_WORLD_SIZE)."""
     if sndbuf < 0:
         sndbuf = loopback_sndbuf(len(os.sched_getaffinity(0)) // max(1, int(os.environ.get("LOCAL_WORLD_SIZE", "1"))))
+    if "NCCL_DYNAMIC_CHUNK_SIZE" not in os.environ:
+        os.environ.setdefault("NCCL_GPUDIRECTTCPX_ENGINE_LEAST_CHUNK", str(128 << 10))
     for k, v in {
         "NCCL_GPUDIRECTTCPX_SOCKET_SNDBUF": str(sndbuf),
         "NCCL_GPUDIRECTTCPX_SOCKET_IFNAME": "lo",

@@ -158,3 +158,17 @@ def test_engine_learns_how_many_ranks_share_the_box():
                                tcpxb_engine_set_local_ranks=lambda h, n: told.append(n) or 0)
     eng._connect()
     assert told == [3]
+
+
+def test_engine_keeps_to_a_quantum_that_the_environment_sets(monkeypatch):
+    """The defaults cut the engine's requests down to 128 KiB; a NCCL_DYNAMIC_CHUNK_SIZE of the caller's own is left alone,
+    and so is the choice not to cut."""
+    import os
+    from nccl_plugin_gpudirecttcpx_b200.parallel.engine import default_transport_env
+    quantum, least = "NCCL_DYNAMIC_CHUNK_SIZE", "NCCL_GPUDIRECTTCPX_ENGINE_LEAST_CHUNK"
+    for given, want in (({}, ("524288", "131072")), ({quantum: "524288"}, ("524288", None)), ({least: "0"}, ("524288", "0")),
+                        ({quantum: "262144", least: "65536"}, ("262144", "65536"))):
+        with monkeypatch.context() as m:
+            m.setattr(os, "environ", dict(given))
+            default_transport_env(sndbuf=0)
+            assert (os.environ[quantum], os.environ.get(least)) == want
