@@ -475,8 +475,10 @@ struct Cfg {
   static_assert(kSmemBytes + 1024 <= 227 * 1024, "slot rings must fit one CTA's shared memory");
 };
 
+// At most 80 registers per thread, as for two CTAs per SM, although the slot rings leave room for one: a CTA of another
+// kernel has to fit beside one that waits for its producer, 1024 threads of 32 registers included (stage_out_kernel).
 template <int RED, bool L2RED, int FAN>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 2)
 unpack_kernel(const __grid_constant__ UnpackParams p) {
   using C = Cfg<RED, L2RED, FAN>;
   extern __shared__ __align__(1024) uint8_t smem[];
