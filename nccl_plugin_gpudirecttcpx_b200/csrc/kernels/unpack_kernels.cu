@@ -921,29 +921,27 @@ stage_out_kernel(const uint8_t* src, uint8_t* dst, uint64_t bytes, uint32_t* fla
 }
 
 // out[i] = sum_r srcs[r][shard_off + i], fp32 adds.
+constexpr int kMaxSources = TCPXB_MAX_PEERS + 1;
 struct PeerReduceParams {
-  const uint8_t* srcs[TCPXB_MAX_PEERS + 1];
-  int nsrcs;
+  const uint8_t* srcs[kMaxSources];
   uint8_t* out;
   uint64_t shard_off;
   uint64_t vecs;
 };
 // Sum of one vector of every source, in the order of the sources.
 template <int RED, int N>
-__device__ __forceinline__ uint4 sum_sources(const uint4 (&v)[N], int n) {
+__device__ __forceinline__ uint4 sum_sources(const uint4 (&v)[N]) {
   if (RED == TCPXB_BF16) {
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
 #pragma unroll
     for (int r = 0; r < N; ++r) {
-      if (r < n) {
-        const uint32_t w[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+      const uint32_t w[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[2 * j] += __uint_as_float(w[j] << 16);
-          acc[2 * j + 1] += __uint_as_float(w[j] & 0xffff0000u);
-        }
+      for (int j = 0; j < 4; ++j) {
+        acc[2 * j] += __uint_as_float(w[j] << 16);
+        acc[2 * j + 1] += __uint_as_float(w[j] & 0xffff0000u);
       }
     }
     uint32_t o[4];
@@ -957,21 +955,20 @@ __device__ __forceinline__ uint4 sum_sources(const uint4 (&v)[N], int n) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int r = 0; r < N; ++r) {
-    if (r < n) {
-      acc.x += __uint_as_float(v[r].x); acc.y += __uint_as_float(v[r].y);
-      acc.z += __uint_as_float(v[r].z); acc.w += __uint_as_float(v[r].w);
-    }
+    acc.x += __uint_as_float(v[r].x); acc.y += __uint_as_float(v[r].y);
+    acc.z += __uint_as_float(v[r].z); acc.w += __uint_as_float(v[r].w);
   }
   return make_uint4(__float_as_uint(acc.x), __float_as_uint(acc.y), __float_as_uint(acc.z), __float_as_uint(acc.w));
 }
 
 // Bound by HBM (or NVLink, for peers' memory).  A thread sums 32 bytes of every source where all addresses allow it
-// (WIDE), 16 otherwise; as many CTAs as that takes, so that no round of a persistent grid is part-filled.  N: the
-// most sources this variant takes; registers for unused ones would cost warps in flight (48 against 96).
-// Measured inside CUDA graphs, four bf16 sources of 16 MiB: 13.9 us with 16-byte loads in a persistent grid of
-// 8 x 256 threads per SM, 13.5 us this way (0.94 of the copy rate).
+// (WIDE), 16 otherwise; as many CTAs as that takes, so that no round of a persistent grid is part-filled.  One variant
+// per number of sources N: registers for absent ones would cost warps in flight, predicates on a number that only the
+// launch knows cost load slots.  Measured inside CUDA graphs, 16-byte loads in a persistent grid of 8 x 256 threads per SM ->
+// this, out of HBM and (in brackets) out of L2: four bf16 sources of 16 MiB 14.5 -> 13.4 us (8.0 -> 6.4), 0.95 of the
+// copy rate; eight fp32 ones of 4 MiB 7.5 -> 6.9 (3.6 -> 3.3); five of 16 MiB 16.4 -> 15.7 (11.4 -> 11.0), where one
+// variant for up to nine took 17.6 (14.7).
 constexpr int kPeerThreads = 256;
-constexpr int kFewSources = 4;
 template <int RED, int N, bool WIDE>
 __global__ void __launch_bounds__(kPeerThreads) peer_reduce_kernel(const __grid_constant__ PeerReduceParams p) {
   const uint64_t i = ((uint64_t)blockIdx.x * kPeerThreads + threadIdx.x) * (WIDE ? 2 : 1);
@@ -983,18 +980,31 @@ __global__ void __launch_bounds__(kPeerThreads) peer_reduce_kernel(const __grid_
     uint4 lo[N], hi[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) {
-      if (r < p.nsrcs) { const Vec32 v = ld_v8(p.srcs[r] + off); lo[r] = v.lo; hi[r] = v.hi; }
+      const Vec32 v = ld_v8(p.srcs[r] + off);
+      lo[r] = v.lo;
+      hi[r] = v.hi;
     }
-    const Vec32 o = {sum_sources<RED, N>(lo, p.nsrcs), sum_sources<RED, N>(hi, p.nsrcs)};
+    __syncwarp(__activemask());  // keeps the adds behind all of the loads: the compiler would wait for the first source first
+    const Vec32 o = {sum_sources<RED, N>(lo), sum_sources<RED, N>(hi)};
     st_v8(p.out + (i << 4), o);
     return;
   }
   uint4 v[N];
 #pragma unroll
-  for (int r = 0; r < N; ++r) {
-    if (r < p.nsrcs) v[r] = ld_v4(p.srcs[r] + off);
-  }
-  *reinterpret_cast<uint4*>(p.out + (i << 4)) = sum_sources<RED, N>(v, p.nsrcs);
+  for (int r = 0; r < N; ++r) v[r] = ld_v4(p.srcs[r] + off);
+  __syncwarp(__activemask());
+  *reinterpret_cast<uint4*>(p.out + (i << 4)) = sum_sources<RED, N>(v);
+}
+
+using PeerReduceKernel = void (*)(PeerReduceParams);
+template <int RED, int N>
+PeerReduceKernel peerReduceKernelFrom(int nsrcs, bool wide) {
+  if (nsrcs == N) return wide ? peer_reduce_kernel<RED, N, true> : peer_reduce_kernel<RED, N, false>;
+  if constexpr (N < kMaxSources) return peerReduceKernelFrom<RED, N + 1>(nsrcs, wide);
+  return nullptr;
+}
+PeerReduceKernel peerReduceKernel(int dtype, int nsrcs, bool wide) {
+  return dtype == TCPXB_BF16 ? peerReduceKernelFrom<TCPXB_BF16, 1>(nsrcs, wide) : peerReduceKernelFrom<TCPXB_F32, 1>(nsrcs, wide);
 }
 
 // Checksum: per-block partial sums into scratch; the last block to arrive adds them.
@@ -1315,11 +1325,9 @@ int tcpxb_kernels_preload(void) {
   signal_flags_kernel<<<1, 32, 0, s>>>(sp);
   PeerReduceParams pp;
   memset(&pp, 0, sizeof pp);
-#define TCPXB_DRY_PEER(RED, N) \
-  peer_reduce_kernel<RED, N, true><<<1, kPeerThreads, 0, s>>>(pp); peer_reduce_kernel<RED, N, false><<<1, kPeerThreads, 0, s>>>(pp)
-  TCPXB_DRY_PEER(TCPXB_BF16, kFewSources); TCPXB_DRY_PEER(TCPXB_BF16, TCPXB_MAX_PEERS + 1);
-  TCPXB_DRY_PEER(TCPXB_F32, kFewSources); TCPXB_DRY_PEER(TCPXB_F32, TCPXB_MAX_PEERS + 1);
-#undef TCPXB_DRY_PEER
+  for (int n = 1; n <= kMaxSources; ++n)
+    for (const int dtype : {TCPXB_BF16, TCPXB_F32})
+      for (const bool wide : {false, true}) peerReduceKernel(dtype, n, wide)<<<1, kPeerThreads, 0, s>>>(pp);
   // The checksum kernel and the address of the allocation-free entry point's scratch:
   // one launch over zero bytes, its result written into the scratch itself, so that
   // the first real tcpxb_checksum_noalloc on this device only clears and launches.
@@ -1494,7 +1502,6 @@ int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_of
       return fail(TCPXB_K_INVALID, "null or misaligned source");
     p.srcs[i] = static_cast<const uint8_t*>(srcs[i]);
   }
-  p.nsrcs = nsrcs;
   p.out = static_cast<uint8_t*>(out);
   p.shard_off = shard_off;
   p.vecs = bytes >> 4;
@@ -1504,12 +1511,7 @@ int tcpxb_peer_reduce(void* out, void* const* srcs, int nsrcs, uint64_t shard_of
   const bool wide = (at & 31) == 0;
   const uint64_t ctas = ((wide ? (p.vecs + 1) / 2 : p.vecs) + kPeerThreads - 1) / kPeerThreads;
   if (ctas > 0x7fffffffull) return fail(TCPXB_K_INVALID, "span beyond the largest grid");
-  const bool bf = dtype == TCPXB_BF16, few = nsrcs <= kFewSources;
-#define TCPXB_PEER(RED, N) (wide ? peer_reduce_kernel<RED, N, true> : peer_reduce_kernel<RED, N, false>)
-  return launchDependent(bf ? (few ? TCPXB_PEER(TCPXB_BF16, kFewSources) : TCPXB_PEER(TCPXB_BF16, TCPXB_MAX_PEERS + 1))
-                            : (few ? TCPXB_PEER(TCPXB_F32, kFewSources) : TCPXB_PEER(TCPXB_F32, TCPXB_MAX_PEERS + 1)),
-                         (unsigned)ctas, kPeerThreads, 0, static_cast<cudaStream_t>(stream), p);
-#undef TCPXB_PEER
+  return launchDependent(peerReduceKernel(dtype, nsrcs, wide), (unsigned)ctas, kPeerThreads, 0, static_cast<cudaStream_t>(stream), p);
 }
 
 size_t tcpxb_checksum_scratch_bytes(void) { return sizeof(CsumScratch); }

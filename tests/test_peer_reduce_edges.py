@@ -30,3 +30,20 @@ def test_edges(dtype, nsrcs, vecs, off):
     assert torch.equal(out.cpu(), want.to(dtype))
     behind = whole[(per if off else 0) + n:]
     assert (behind == 5.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("nsrcs", range(1, 10))
+@pytest.mark.parametrize("vecs", [3, 514])
+def test_every_number_of_sources(dtype, nsrcs, vecs):
+    """One kernel each; an odd last vector and whole 32-byte pairs, on and off the 32-byte phase."""
+    per = 16 // dtype.itemsize
+    g = torch.Generator().manual_seed(nsrcs)
+    srcs = [torch.randn((vecs + 2) * per, generator=g).to(dtype) for _ in range(nsrcs)]
+    for off in (0, 1):
+        out = torch.empty(vecs * per, dtype=dtype, device="cuda")
+        ops.peer_reduce(out, [s.cuda() for s in srcs], shard_off=off * 16)
+        want = torch.zeros(vecs * per)
+        for s in srcs:
+            want = want + s[off * per:off * per + vecs * per].float()
+        assert torch.equal(out.cpu(), want.to(dtype))
