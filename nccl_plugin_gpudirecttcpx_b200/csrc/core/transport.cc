@@ -533,8 +533,9 @@ Result startCudaSend(Comm* comm, Request* r, MemHandle* mh) {
     }
     return kSuccess;
   }
-  // One staging copy per ~2 MiB: enough to let the first chunks leave while the
-  // rest is still being copied, few enough that the per-copy launch cost stays small.
+  // One staging copy per ~2 MiB: from 4 MiB on the first chunks leave while the rest is still
+  // being copied, and the copies stay few enough for their launch cost.  Smaller sends, the
+  // collective engine's 1 MiB requests among them, are one copy.
   const int chunk = chunkBytesFor(r->size, comm->num_socks, comm->least_chunk);
   int n_want = std::max(1, std::min(kMaxTxSegments, r->size / (2 << 20)));
   int seg = (r->size + n_want - 1) / n_want;

@@ -119,7 +119,7 @@ struct Engine {
   uint32_t* ticket = nullptr;       // fan-out completion counter (device)
   uint32_t* status_host = nullptr;  // kernel status block (pinned, device-mapped)
   uint32_t* status_dev = nullptr;
-  gpu::StreamCounter kernel_marks;  // advanced on the caller's stream behind every unpack launch
+  gpu::StreamCounter kernel_marks;  // advanced by every unpack launch at its end (in plain_mode on the stream, behind it)
   gpu::Event dep_event = nullptr;
   tcpxbEngineStats stats;
   int req_bytes = 1 << 20, inflight = 4, ctas = 16;
@@ -291,8 +291,9 @@ int launchUnpack(Engine* e, Request* req, const RecvSpec& rs, uint64_t region_of
   opts.ticket = e->ticket;
   uint32_t* done = e->kernel_marks.take(done_mark);
   const bool nvls = fan && e->cfg.use_nvls && e->mc_out != nullptr;
+  const int impl = !fan && acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM;
   ENG_K(tcpxb_unpack_request(sl.pool_dev, sl.pool_bytes, acc, dst, nvls ? e->mc_out + rs.out_offset + region_off : nullptr, len, peers,
-                             npeers, descs, reinterpret_cast<const tcpxbLoadMeta*>(sl.host), count, rs.dtype, !fan && acc == dst ? e->cfg.reduce_impl : TCPXB_REDUCE_SM, e->status_dev,
+                             npeers, descs, reinterpret_cast<const tcpxbLoadMeta*>(sl.host), count, rs.dtype, impl, e->status_dev,
                              &opts, done, *done_mark, stream));
   return 0;
 }

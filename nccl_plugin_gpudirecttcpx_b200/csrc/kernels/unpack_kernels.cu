@@ -1181,12 +1181,18 @@ int launch(const UnpackParams& p, int max_ctas, cudaStream_t stream) {
   if constexpr (FAN == FAN_NONE && !L2RED) {
     // Up to one record per ring warp the ring kernel is ahead (4 MiB in pages: 2.4 against 3.2 us, its bulk
     // copies need one instruction per page); beyond that its second, part-filled round costs more than it saves.
+    // Ring -> register kernel, buffers out of HBM: 1777 whole pages copied 4.8 -> 4.5 us, summed 6.6 -> 5.4; 3000 of 1448
+    // bytes copied 4.1 -> 3.4, summed 5.1 -> 4.3; 16384 pages 24.6 -> 23.3 and 34.0 -> 31.9.  Where the ring stays ahead: whole
+    // pages copied within L2 (3000: 3.7 -> 4.4), 5000 to 10000 copies of 1448 to 3000 bytes (up to 10 %).  A pool in pinned
+    // host memory, 8 MiB: pages 169 -> 167 us, sums of 1448-byte fragments 178 -> 184, copies of them 176 -> 186 (their edges are
+    // read twice over PCIe); packing from HBM into host memory 172 -> 170.  Telling host memory apart would cost every
+    // launch a driver query of half a microsecond.
     // A launch confined to a few CTAs, streamed or asked to publish its completion stays with the ring.
     if (whole_gpu && p.ready == nullptr && p.flag_value == 0 && p.done_flag == nullptr && p.count > (uint32_t)(sms * kWarps))
       return launchDependent(unpack_wide_kernel<RED>, (p.count + kWideWarps - 1) / kWideWarps, kWideThreads, 0, stream, p);
   }
   // As many SMs as there are records before any SM gets a second one: a record is one warp's work, and 12 of
-  // them on one SM share its bulk-copy engine (256 records: 3.1 us on 22 SMs, 2.3 us on 148).
+  // them on one SM share its bulk-copy engine (256 records: 3.1 us on 22 SMs, 1.9 us on 148).
   const int cap = whole_gpu ? sms : max_ctas;
   const int ctas = p.count < (uint32_t)cap ? (int)p.count : cap;
   UnpackParams q = p;
